@@ -140,7 +140,7 @@ Layout make_layout(const paces_ctx* c, int64_t cap) {
     l.v_TA = take(ucap * cs);
     l.v_TB = take(ucap * cs);
     l.v_partials = take(size_t(2) * c->taylor_grid * 4 * 8);
-    l.v_bar = take(16);
+    l.v_bar = take(kTaylorBarrierBytes);
     l.o_partials = take(size_t(obs_max_grid(c->num_sms)) * (4 + 2 * L) * 8);
     l.o_out = take(size_t(3 + 2 * L) * 8);
     l.aw = take((ucap + 1) * 4);
@@ -227,6 +227,7 @@ TaylorWs taylor_ws(const paces_ctx* c, const Layout& l, void* ws) {
     w.tb = at<void>(ws, l.v_TB);
     w.partials = at<double>(ws, l.v_partials);
     w.barrier = at<unsigned>(ws, l.v_bar);
+    w.maxima = at<unsigned long long>(ws, l.v_bar + kTaylorMaximaOffset);
     w.wait_ns = c->test_wait_ns ? c->test_wait_ns : kWaitLimitNs;
     w.skip_block = c->test_skip_block;
     w.diag = nullptr;

@@ -1,14 +1,16 @@
-// Bounded grid-wide barrier of the persistent cooperative kernels (the Taylor series).
+// Bounded grid-wide barrier of the persistent cooperative kernels (the propagators).
 #pragma once
 
 #include "common.cuh"
 
 namespace paces {
 
-// All blocks are co-resident (cooperative launch).  bar[0] counts arrivals, bar[1] is the
-// generation; a wait longer than `limit_ns` raises PACES_ERR_TIMEOUT on `status` (if given)
-// and returns false instead of spinning on.  `skip` (a test hook) makes this block give up
-// without arriving: it raises the timeout itself, and every other block's wait runs out.
+// All blocks are co-resident (cooperative launch).  bar[0] counts arrivals over all barriers of
+// the launch (zeroed before it); barrier `gen` is passed when it reaches (gen + 1) * nblocks, so
+// an arrival is one atomic and a waiting block only reads.  A wait longer than `limit_ns` raises
+// PACES_ERR_TIMEOUT on `status` (if given) and returns false instead of spinning on.  `skip` (a
+// test hook) makes this block give up without arriving: it raises the timeout itself, and every
+// other block's wait runs out.
 __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, unsigned& gen, int* status,
                                              uint64_t limit_ns = kWaitLimitNs, bool skip = false) {
     __shared__ int s_ok;
@@ -17,27 +19,25 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned nblocks, un
         raise_status(status, PACES_ERR_TIMEOUT);
         s_ok = 0;
     } else if (threadIdx.x == 0) {
-        s_ok = 1;
+        int ok = 1;
+        const unsigned target = (gen + 1) * nblocks;
         __threadfence();
-        const unsigned arrived = atomicAdd(&bar[0], 1u);
-        if (arrived == nblocks - 1) {
-            atomicExch(&bar[0], 0u);
-            __threadfence();
-            atomicAdd(&bar[1], 1u);
-        } else {
-            const uint64_t t0 = global_ns();
-            while (atomicAdd(&bar[1], 0u) == gen) {
-                if (global_ns() - t0 > limit_ns) {
-                    raise_status(status, PACES_ERR_TIMEOUT);
-                    s_ok = 0;
-                    break;
-                }
-                __nanosleep(32);
+        atomicAdd(bar, 1u);
+        const uint64_t t0 = global_ns();
+        unsigned seen;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+            if (int(seen - target) >= 0) break;
+            if (global_ns() - t0 > limit_ns) {
+                raise_status(status, PACES_ERR_TIMEOUT);
+                ok = 0;
+                break;
             }
         }
-        ++gen;
         __threadfence();
+        s_ok = ok;
     }
+    ++gen;
     __syncthreads();
     return s_ok != 0;
 }

@@ -48,11 +48,14 @@ struct TaylorWs {
     void* ta;            // [cap] complex
     void* tb;            // [cap] complex
     double* partials;    // [2][max_grid][4]
-    unsigned* barrier;   // [2]
+    unsigned* barrier;   // grid_barrier's counter, and maxima behind it: kTaylorBarrierBytes, zeroed per launch
+    unsigned long long* maxima;  // [3][4] a sweep's maxima (fp64 bit patterns), the buffers in rotation
     uint64_t wait_ns;    // grid-barrier wait limit (kWaitLimitNs unless a test shortens it)
     int skip_block;      // test hook: this block skips its first grid-barrier arrival (-1: none)
     double* diag;        // null, or [diag_groups(rows)][3]: see diag_group
 };
+constexpr size_t kTaylorMaximaOffset = 64;
+constexpr size_t kTaylorBarrierBytes = kTaylorMaximaOffset + 3 * 4 * 8;
 int taylor_max_grid(bool c64, int num_sms);
 
 // ---- diagnostics of the input state, from the first Taylor sweep ---------------------------

@@ -15,11 +15,23 @@
 // Two row schedules (a tuning choice; the results are identical because every row's
 // arithmetic is the same and the maxima are exact):
 //  * direct: grid-stride, two rows per thread per pass, all loads from global memory;
-//  * bulk:   each block owns 512-row chunks; while it computes one chunk, one thread has
-//            the next chunk's neighbour rows, metadata, result and own term elements
-//            brought into the other half of a shared-memory double buffer by bulk TMA
-//            copies (cp.async.bulk, completion on an mbarrier), so the streaming reads are
-//            in flight while the gathers of the current chunk wait on L2.
+//  * bulk:   each block owns 512-row chunks.  When no block owns more than two, they stay in
+//            shared memory for the whole series: a sweep then only gathers, stores the new
+//            term and updates the sum on chip (S up to 1024 rows per block of the wave).
+//            Otherwise the chunks stream: while a block computes one, one thread has the
+//            next chunk's neighbour rows, metadata and own elements brought into the other
+//            half of a shared-memory double buffer by bulk TMA copies (cp.async.bulk,
+//            completion on an mbarrier), so the streaming reads are in flight while the
+//            gathers of the current chunk wait on L2.
+//
+// The streamed sum lags: a sweep that starts with the sum up to date writes its term only,
+// and the next one adds both terms in the order of the series (the row's own element of the
+// source is the last term, and it is loaded for H's diagonal anyway).  Per pair of sweeps the
+// sum is read and written once instead of twice.  The stop test needs the sum's inf-norm; in
+// a sweep that left the sum alone it is known to lie within the new term's norm of the last
+// exact one, which settles the test unless the series may end here -- then an extra pass adds
+// the term and measures the norm.  Terms, sums, norms and decisions are the ones of a series
+// that updates the sum in every sweep, bit for bit.
 #include "grid.cuh"
 #include "hrow.cuh"
 #include "kernels.cuh"
@@ -32,22 +44,47 @@ namespace {
 constexpr int kTThreads = 256;
 constexpr int kTWarps = kTThreads / 32;
 
-// max-reduce four values over the block; result in out[0..3] (shared), valid after return.
-__device__ void block_max4(double v[4], double (*red)[kTWarps], double* out) {
+// Largest of a warp's non-negative values (their bit patterns order like the values).
+__device__ __forceinline__ float warp_max(float v) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ double warp_max(double v) {
+    const unsigned hi = unsigned(__double2hiint(v)), lo = unsigned(__double2loint(v));
+    const unsigned h = __reduce_max_sync(0xffffffffu, hi);
+    return __hiloint2double(int(h), int(__reduce_max_sync(0xffffffffu, hi == h ? lo : 0u)));
+}
+
+// A sweep's maxima over the grid: |term|^2, |res|^2, |v|^2 (first sweep) and a non-finite flag.
+template <typename R>
+struct SweepMax {
+    R term, res, v;
+    bool bad;
+};
+
+// Fold the block's maxima into g[0..3] (fp64 bit patterns; atomicMax is exact and order-free),
+// pass the grid barrier and read the grid's maxima into fin[0..3] (shared).  false on a timeout.
+template <typename R>
+__device__ bool grid_max(const SweepMax<R>& mx, unsigned long long* g, double (*red)[kTWarps], double* fin,
+                         const TaylorWs& ws, unsigned& gen, int* status) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] = fmax(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-        if (lane == 0) red[k][wid] = v[k];
+    const R a = warp_max(mx.term), b = warp_max(mx.res), c = warp_max(mx.v);
+    const bool bad = __any_sync(0xffffffffu, mx.bad);
+    if (lane == 0) {
+        red[0][wid] = double(a);
+        red[1][wid] = double(b);
+        red[2][wid] = double(c);
+        red[3][wid] = bad ? 1.0 : 0.0;
     }
     __syncthreads();
     if (threadIdx.x < 4) {
         double r = 0.0;
         for (int w = 0; w < kTWarps; ++w) r = fmax(r, red[threadIdx.x][w]);
-        out[threadIdx.x] = r;
+        if (r > 0.0) atomicMax(g + threadIdx.x, static_cast<unsigned long long>(__double_as_longlong(r)));
     }
+    if (!grid_barrier(ws.barrier, gridDim.x, gen, status, ws.wait_ns, int(blockIdx.x) == ws.skip_block)) return false;
+    if (threadIdx.x < 4) fin[threadIdx.x] = __longlong_as_double((long long)__ldcg(g + threadIdx.x));
     __syncthreads();
+    return true;
 }
 
 constexpr int kChunk = 2 * kTThreads;  // rows per block pass of the bulk schedule
@@ -83,7 +120,6 @@ taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ n
     uint32_t pending = 0;   // bulk, thread 0: buffers with copies issued and not yet consumed
 
     const int64_t S = blk[m.L];
-    const unsigned nblocks = gridDim.x;
     unsigned gen = 0;
     const C* v = reinterpret_cast<const C*>(v_in);
     C* res = reinterpret_cast<C*>(res_out);
@@ -93,13 +129,74 @@ taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ n
     double c1 = 0.0, c1c2 = 0.0, ratio = 0.0;
     int conv = 0, fin_j = 0;
 
+    // bulk: the chunks this block owns (c, c + grid, ..); with at most two they stay in the two
+    // buffers for the whole series, otherwise they stream through them
+    const int64_t nch = (S + kChunk - 1) / kChunk;
+    const bool resident = BULK && nch <= 2 * int64_t(gridDim.x);
+    // bulk, streaming: the sum lags one term behind (see the head of this file)
+    bool lag = false;
+    const C* rbase = v;      // where the sum without the lagging term is
+    double rnorm = 0.0;      // its inf-norm
+    unsigned sweep = 0;      // barriers passed with maxima: the maxima's buffers rotate
+    auto maxima = [&](unsigned s) { return ws.maxima + (s % 3) * 4; };
+    // after sweep s's barrier: clear the buffer that sweep s + 2 folds into
+    auto next_sweep = [&]() {
+        if (blockIdx.x == 0 && threadIdx.x < 4) maxima(sweep + 2)[threadIdx.x] = 0ull;
+        ++sweep;
+    };
+    constexpr uint32_t kCB = chunk_bytes<C64>();
+    constexpr uint32_t kOffMeta = kChunk * 16, kOffRin = kOffMeta + kChunk * 4,
+                       kOffSelf = kOffRin + kChunk * sizeof(C);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // chunk rows of this thread when a warp holds one 64-row group (the first sweep's diagnostics)
+    const int g0 = kDiagGroup * wid + lane, g1 = g0 + 32;
+    if constexpr (BULK) {
+        if (resident) {
+            for (int k = 0; k < 2; ++k) {
+                const int64_t r0 = (blockIdx.x + int64_t(k) * gridDim.x) * kChunk;
+                unsigned char* base = t_smem + k * kCB;
+                for (int t = threadIdx.x; t < kChunk && r0 + t < S; t += kTThreads) {
+                    reinterpret_cast<int4*>(base)[t] = load_nbr(nbr, r0 + t);
+                    reinterpret_cast<uint32_t*>(base + kOffMeta)[t] = __ldg(meta + r0 + t);
+                    const C z = v[r0 + t];
+                    reinterpret_cast<C*>(base + kOffRin)[t] = z;
+                    reinterpret_cast<C*>(base + kOffSelf)[t] = z;
+                }
+            }
+            __syncthreads();
+        }
+    }
+
     for (int j = 0; j < m_star; ++j) {
         const C* src = j == 0 ? v : ((j & 1) ? ta : tb);
         C* dst = (j & 1) ? tb : ta;
-        const C* rin = j == 0 ? v : res;
         const double cd = dt / double(j + 1);
         const R c = R(cd);
-        double mx[4] = {0.0, 0.0, 0.0, 0.0};  // |term|, |res|, |v|, non-finite
+        SweepMax<R> mx{R(0), R(0), R(0), false};
+        auto sq_abs = [](const C& z) -> R {
+            if constexpr (C64) return fmaf(z.x, z.x, __fmul_rn(z.y, z.y));
+            else return fma(z.x, z.x, __dmul_rn(z.y, z.y));
+        };
+        auto finite = [](const C& z) { return isfinite(z.x) && isfinite(z.y); };
+        auto add = [](const C& a, const C& t) -> C {
+            if constexpr (C64) return make_float2(__fadd_rn(a.x, t.x), __fadd_rn(a.y, t.y));
+            else return make_double2(__dadd_rn(a.x, t.x), __dadd_rn(a.y, t.y));
+        };
+        // the new term from y = H src: separate roundings (no contraction into an FMA), so that
+        // every kernel and schedule that runs these rows -- direct, bulk, batched -- rounds alike
+        auto term = [&](const C& y) -> C {
+            C t;
+            if constexpr (C64) t = make_float2(__fmul_rn(c, y.y), -__fmul_rn(c, y.x));
+            else t = make_double2(__dmul_rn(cd, y.y), -__dmul_rn(cd, y.x));
+            mx.term = fmax(mx.term, sq_abs(t));
+            return t;
+        };
+        auto sum_to = [&](const C& a, const C& t) -> C {  // a + t, the new sum
+            const C rr = add(a, t);
+            mx.res = fmax(mx.res, sq_abs(rr));
+            mx.bad |= !finite(rr);
+            return rr;
+        };
         auto hrow = [&](int64_t r) -> C {
             const uint32_t mm = __ldg(meta + r);
             if constexpr (XHOP) {
@@ -110,30 +207,27 @@ taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ n
                 else return h_row_c128(m, s_sq, r, nbr, mm, src);
             }
         };
-        auto finish = [&](int64_t r, const C& y, const C& a) {
-            C t, rr;
-            if constexpr (C64) {
-                // separate roundings (no contraction into an FMA): every kernel and schedule that
-                // runs these rows -- direct, bulk, batched -- must round them alike
-                t = make_float2(__fmul_rn(c, y.y), -__fmul_rn(c, y.x));
-                rr = make_float2(__fadd_rn(a.x, t.x), __fadd_rn(a.y, t.y));
-                mx[0] = fmax(mx[0], double(fmaf(t.x, t.x, __fmul_rn(t.y, t.y))));
-                mx[1] = fmax(mx[1], double(fmaf(rr.x, rr.x, __fmul_rn(rr.y, rr.y))));
-                if (j == 0) mx[2] = fmax(mx[2], double(fmaf(a.x, a.x, __fmul_rn(a.y, a.y))));
+        // one row of a chunk whose neighbour row, metadata and own element are in shared memory
+        auto crow = [&](int64_t r, const int4& nb, uint32_t mm, const C& own) -> C {
+            if constexpr (XHOP) {
+                if constexpr (C64) return h_row_c64_x(m, s_sq, r, nb, mm, own, src);
+                else return h_row_c128_x(m, s_sq, r, nb, mm, own, src);
+            } else if constexpr (C64) {
+                return h_row_c64_nb(m, s_sq, J, r, nb, mm, own, src);
             } else {
-                t = make_double2(__dmul_rn(cd, y.y), -__dmul_rn(cd, y.x));
-                rr = make_double2(__dadd_rn(a.x, t.x), __dadd_rn(a.y, t.y));
-                mx[0] = fmax(mx[0], fma(t.x, t.x, __dmul_rn(t.y, t.y)));
-                mx[1] = fmax(mx[1], fma(rr.x, rr.x, __dmul_rn(rr.y, rr.y)));
-                if (j == 0) mx[2] = fmax(mx[2], fma(a.x, a.x, __dmul_rn(a.y, a.y)));
+                return h_row_c128_nb(m, s_sq, r, nb, mm, own, src);
             }
-            if (!(isfinite(double(rr.x)) && isfinite(double(rr.y)))) mx[3] = 1.0;
-            dst[r] = t;
-            res[r] = rr;
         };
         const bool diag = j == 0 && ws.diag != nullptr;  // first sweep: fold the input's diagnostics
-        const int wid = threadIdx.x >> 5;
+        bool exact = true;  // this sweep brings the sum and its norm up to date
         if constexpr (!BULK) {
+            const C* rin = j == 0 ? v : res;
+            auto finish = [&](int64_t r, const C& y, const C& a) {
+                const C t = term(y);
+                if (j == 0) mx.v = fmax(mx.v, sq_abs(a));
+                res[r] = sum_to(a, t);
+                dst[r] = t;
+            };
             // two rows per thread per pass: all loads of both rows precede the stores
             const int64_t stride = int64_t(gridDim.x) * kTThreads;
             if (!diag) {
@@ -148,7 +242,6 @@ taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ n
             } else {
                 // every row once, in 64-row units per warp (rows u + lane and u + 32 + lane, a
                 // warp-uniform loop), so that each warp folds its 64-row groups
-                const int lane = threadIdx.x & 31;
                 const int64_t ustride = int64_t(gridDim.x) * kTWarps * kDiagGroup;
                 for (int64_t ub = (int64_t(blockIdx.x) * kTWarps + wid) * kDiagGroup; ub < S; ub += ustride) {
                     const int64_t r0 = ub + lane, r1 = ub + 32 + lane;
@@ -167,40 +260,80 @@ taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ n
                     diag_group(ws.diag, ub / kDiagGroup, v0, a0, y0, v1, a1, y1);
                 }
             }
+        } else if (resident) {
+            for (int k = 0; k < 2; ++k) {
+                const int64_t ch = blockIdx.x + int64_t(k) * gridDim.x;
+                const int64_t r0 = ch * kChunk;
+                if (r0 + kDiagGroup * wid >= S) break;  // no row of this warp's group
+                unsigned char* base = t_smem + k * kCB;
+                const int4* snb = reinterpret_cast<const int4*>(base);
+                const uint32_t* smeta = reinterpret_cast<const uint32_t*>(base + kOffMeta);
+                C* sres = reinterpret_cast<C*>(base + kOffRin);
+                C* sself = reinterpret_cast<C*>(base + kOffSelf);
+                const bool v0 = r0 + g0 < S, v1 = r0 + g1 < S;
+                C y0{}, y1{};
+                if (v0) y0 = crow(r0 + g0, snb[g0], smeta[g0], sself[g0]);
+                if (v1) y1 = crow(r0 + g1, snb[g1], smeta[g1], sself[g1]);
+                if (diag) {
+                    const C z{};
+                    diag_group(ws.diag, r0 / kDiagGroup + wid, v0, v0 ? sself[g0] : z, y0, v1, v1 ? sself[g1] : z, y1);
+                }
+                auto finish = [&](int g, const C& y) {
+                    const C t = term(y);
+                    const C a = sres[g];
+                    if (j == 0) mx.v = fmax(mx.v, sq_abs(a));
+                    sres[g] = sum_to(a, t);
+                    sself[g] = t;
+                    dst[r0 + g] = t;
+                };
+                if (v0) finish(g0, y0);
+                if (v1) finish(g1, y1);
+            }
         } else {
-            constexpr uint32_t kCB = chunk_bytes<C64>();
-            constexpr uint32_t kOffMeta = kChunk * 16, kOffRin = kOffMeta + kChunk * 4,
-                               kOffSelf = kOffRin + kChunk * sizeof(C);
-            const int64_t nch = (S + kChunk - 1) / kChunk;
-            auto full = [&](int64_t c) { return (c + 1) * kChunk <= S; };
-            auto issue = [&](int64_t c, int b) {  // thread 0
-                const int64_t r0 = c * kChunk;
+            exact = lag;
+            auto full = [&](int64_t ch) { return (ch + 1) * kChunk <= S; };
+            auto issue = [&](int64_t ch, int b) {  // thread 0
+                const int64_t r0 = ch * kChunk;
                 const uint32_t base = tc::smem_addr(t_smem + b * kCB);
                 const uint32_t mb = tc::smem_addr(&s_mbar[b]);
-                tc::mbar_expect_tx(mb, kCB);
+                tc::mbar_expect_tx(mb, lag ? kCB : kCB - kChunk * uint32_t(sizeof(C)));
                 tc::bulk_g2s(base, nbr + r0 * 4, kChunk * 16, mb);
                 tc::bulk_g2s(base + kOffMeta, meta + r0, kChunk * 4, mb);
-                tc::bulk_g2s(base + kOffRin, rin + r0, kChunk * sizeof(C), mb);
+                if (lag) tc::bulk_g2s(base + kOffRin, rbase + r0, kChunk * sizeof(C), mb);
                 tc::bulk_g2s(base + kOffSelf, src + r0, kChunk * sizeof(C), mb);
                 pending |= 1u << b;
             };
-            int64_t c = blockIdx.x;
-            if (threadIdx.x == 0 && c < nch) {
+            // row r: its new term and, when the sum lags, the sum with the last term and this one
+            auto finish = [&](int64_t r, const C& y, const C& own, const C& a) {
+                const C t = term(y);
+                if (lag) {
+                    const C prev = add(a, own);
+                    mx.bad |= !finite(prev);
+                    res[r] = sum_to(prev, t);
+                } else {
+                    mx.bad |= !finite(t);
+                    if (j == 0) {
+                        mx.bad |= !finite(own);
+                        mx.v = fmax(mx.v, sq_abs(own));
+                    }
+                }
+                dst[r] = t;
+            };
+            int64_t ch = blockIdx.x;
+            if (threadIdx.x == 0 && ch < nch) {
                 // the previous term's stores (every block's, ordered by the grid barrier) before
                 // this term's bulk reads of them
                 tc::fence_proxy_async_global();
-                if (full(c)) issue(c, 0);
+                if (full(ch)) issue(ch, 0);
             }
-            for (int k = 0; c < nch; c += gridDim.x, ++k) {
+            for (int k = 0; ch < nch; ch += gridDim.x, ++k) {
                 const int b = k & 1;
-                const int64_t cn = c + gridDim.x;
+                const int64_t cn = ch + gridDim.x;
                 if (threadIdx.x == 0 && cn < nch && full(cn)) issue(cn, b ^ 1);
-                const int64_t r0 = c * kChunk;
-                // chunk rows of this thread: t and t + 256, or in the first sweep with the
-                // diagnostics 64 w + lane and 64 w + 32 + lane (warp w's 64-row group)
-                const int t0 = diag ? kDiagGroup * wid + (threadIdx.x & 31) : threadIdx.x;
-                const int t1 = diag ? t0 + 32 : threadIdx.x + kTThreads;
-                if (full(c)) {
+                const int64_t r0 = ch * kChunk;
+                const int t0 = diag ? g0 : threadIdx.x;
+                const int t1 = diag ? g1 : threadIdx.x + kTThreads;
+                if (full(ch)) {
                     if (!tc::mbar_wait(tc::smem_addr(&s_mbar[b]), (parity >> b) & 1u)) s_abort = 1;
                     parity ^= 1u << b;
                     if (threadIdx.x == 0) pending &= ~(1u << b);
@@ -209,38 +342,26 @@ taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ n
                     const uint32_t* smeta = reinterpret_cast<const uint32_t*>(base + kOffMeta);
                     const C* srin = reinterpret_cast<const C*>(base + kOffRin);
                     const C* sself = reinterpret_cast<const C*>(base + kOffSelf);
-                    C y0, y1;
-                    if constexpr (XHOP) {
-                        if constexpr (C64) {
-                            y0 = h_row_c64_x(m, s_sq, r0 + t0, snb[t0], smeta[t0], sself[t0], src);
-                            y1 = h_row_c64_x(m, s_sq, r0 + t1, snb[t1], smeta[t1], sself[t1], src);
-                        } else {
-                            y0 = h_row_c128_x(m, s_sq, r0 + t0, snb[t0], smeta[t0], sself[t0], src);
-                            y1 = h_row_c128_x(m, s_sq, r0 + t1, snb[t1], smeta[t1], sself[t1], src);
-                        }
-                    } else if constexpr (C64) {
-                        y0 = h_row_c64_nb(m, s_sq, J, r0 + t0, snb[t0], smeta[t0], sself[t0], src);
-                        y1 = h_row_c64_nb(m, s_sq, J, r0 + t1, snb[t1], smeta[t1], sself[t1], src);
-                    } else {
-                        y0 = h_row_c128_nb(m, s_sq, r0 + t0, snb[t0], smeta[t0], sself[t0], src);
-                        y1 = h_row_c128_nb(m, s_sq, r0 + t1, snb[t1], smeta[t1], sself[t1], src);
-                    }
-                    finish(r0 + t0, y0, srin[t0]);
-                    finish(r0 + t1, y1, srin[t1]);
-                    if (diag) diag_group(ws.diag, r0 / kDiagGroup + wid, true, srin[t0], y0, true, srin[t1], y1);
+                    const C y0 = crow(r0 + t0, snb[t0], smeta[t0], sself[t0]);
+                    const C y1 = crow(r0 + t1, snb[t1], smeta[t1], sself[t1]);
+                    const C z{};
+                    finish(r0 + t0, y0, sself[t0], lag ? srin[t0] : z);
+                    finish(r0 + t1, y1, sself[t1], lag ? srin[t1] : z);
+                    if (diag) diag_group(ws.diag, r0 / kDiagGroup + wid, true, sself[t0], y0, true, sself[t1], y1);
                 } else {
                     // the last, partial chunk: direct loads
                     const bool v0 = r0 + t0 < S, v1 = r0 + t1 < S;
                     C y0{}, y1{}, a0{}, a1{};
+                    const C z{};
                     if (v0) {
                         y0 = hrow(r0 + t0);
-                        a0 = rin[r0 + t0];
-                        finish(r0 + t0, y0, a0);
+                        a0 = __ldcg(src + r0 + t0);
+                        finish(r0 + t0, y0, a0, lag ? rbase[r0 + t0] : z);
                     }
                     if (v1) {
                         y1 = hrow(r0 + t1);
-                        a1 = rin[r0 + t1];
-                        finish(r0 + t1, y1, a1);
+                        a1 = __ldcg(src + r0 + t1);
+                        finish(r0 + t1, y1, a1, lag ? rbase[r0 + t1] : z);
                     }
                     if (diag && r0 + kDiagGroup * wid < S)  // groups with at least one row (warp-uniform)
                         diag_group(ws.diag, r0 / kDiagGroup + wid, v0, a0, y0, v1, a1, y1);
@@ -258,26 +379,9 @@ taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ n
                 break;
             }
         }
-        block_max4(mx, s_red, s_fin);
-        if (threadIdx.x == 0) {
-            double* pp = ws.partials + (size_t((j & 1) * nblocks) + blockIdx.x) * 4;
-            pp[0] = s_fin[0];
-            pp[1] = s_fin[1];
-            pp[2] = s_fin[2];
-            pp[3] = s_fin[3];
-        }
-        if (!grid_barrier(ws.barrier, nblocks, gen, status, ws.wait_ns, int(blockIdx.x) == ws.skip_block)) {
-            fin_j = j;
-            break;
-        }
-        double g4[4] = {0.0, 0.0, 0.0, 0.0};
-        for (unsigned b = threadIdx.x; b < nblocks; b += kTThreads) {
-            const double* pp = ws.partials + (size_t((j & 1) * nblocks) + b) * 4;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) g4[k] = fmax(g4[k], __ldcg(pp + k));
-        }
-        block_max4(g4, s_red, s_fin);
         fin_j = j;
+        if (!grid_max(mx, maxima(sweep), s_red, s_fin, ws, gen, status)) break;
+        next_sweep();
         if (s_fin[3] != 0.0) {
             if (blockIdx.x == 0 && threadIdx.x == 0) raise_status(status, PACES_ERR_NONFINITE);
             break;
@@ -286,12 +390,62 @@ taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ n
         if (j == 0) c1 = sqrt(s_fin[2]);
         const double c2 = sqrt(s_fin[0]);
         c1c2 = c1 + c2;
-        ratio = c1c2 / sqrt(s_fin[1]);
-        if (ratio <= tol) {
-            conv = 1;
-            break;
+        if (exact) {
+            if (lag) rbase = res;
+            lag = false;
+            rnorm = sqrt(s_fin[1]);
+        } else {
+            if (j == 0) rnorm = c1;
+            lag = true;
+            // the sum's norm lies in rnorm -+ c2 (to a few roundings): only a ratio that may end
+            // the series, or the series' last, needs it exactly
+            if (j == m_star - 1 || c1c2 <= tol * (rnorm + c2) * 1.00001) {
+                mx = SweepMax<R>{R(0), R(0), R(0), false};
+                for (int64_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+                    const int64_t r0 = ch * kChunk + threadIdx.x, r1 = r0 + kTThreads;
+                    C a0{}, a1{}, b0{}, b1{};
+                    if (r0 < S) {
+                        a0 = __ldcg(rbase + r0);
+                        b0 = __ldcg(dst + r0);
+                    }
+                    if (r1 < S) {
+                        a1 = __ldcg(rbase + r1);
+                        b1 = __ldcg(dst + r1);
+                    }
+                    if (r0 < S) res[r0] = sum_to(a0, b0);
+                    if (r1 < S) res[r1] = sum_to(a1, b1);
+                }
+                if (!grid_max(mx, maxima(sweep), s_red, s_fin, ws, gen, status)) break;
+                next_sweep();
+                if (s_fin[3] != 0.0) {
+                    if (blockIdx.x == 0 && threadIdx.x == 0) raise_status(status, PACES_ERR_NONFINITE);
+                    break;
+                }
+                exact = true;
+                rbase = res;
+                lag = false;
+                rnorm = sqrt(s_fin[1]);
+            }
+        }
+        if (exact) {
+            ratio = c1c2 / rnorm;
+            if (ratio <= tol) {
+                conv = 1;
+                break;
+            }
         }
         c1 = c2;
+    }
+    if constexpr (BULK) {
+        if (resident) {
+            // the sum out of shared memory (each thread its own rows)
+            for (int k = 0; k < 2; ++k) {
+                const int64_t r0 = (blockIdx.x + int64_t(k) * gridDim.x) * kChunk;
+                const C* sres = reinterpret_cast<const C*>(t_smem + k * kCB + kOffRin);
+                if (r0 + g0 < S) res[r0 + g0] = sres[g0];
+                if (r0 + g1 < S) res[r0 + g1] = sres[g1];
+            }
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (out.converged) *out.converged = conv;
@@ -356,12 +510,12 @@ int launch_taylor(bool c64, const ModelDev& m, const int* blk, const int* nbr, i
                   int blocks_per_sm, int variant, cudaStream_t st) {
     if (m_star < 1 || variant < 0 || variant > 1) return PACES_ERR_BADARG;
     if (m.nhop > 1 && !m.xnbr) return PACES_ERR_BADARG;
-    if (cudaMemsetAsync(ws.barrier, 0, 2 * sizeof(unsigned), st) != cudaSuccess) return PACES_ERR_CUDA;
+    if (cudaMemsetAsync(ws.barrier, 0, kTaylorBarrierBytes, st) != cudaSuccess) return PACES_ERR_CUDA;
     const bool xhop = m.nhop > 1;
     const int occ = c64 ? occupancy_any<true>(variant, xhop) : occupancy_any<false>(variant, xhop);
-    // a wave of blocks, or one block per 2048 rows of a small problem (fewer blocks at the grid
-    // barriers; the results do not depend on the grid)
-    const int grid = grid_for(nbr_cap, 2048, num_sms * (blocks_per_sm > 0 && blocks_per_sm < occ ? blocks_per_sm : occ));
+    // a wave of blocks, or one block per 1024 rows of room in a small problem (fewer blocks at the
+    // grid barriers, and at most two chunks each; the results do not depend on the grid)
+    const int grid = grid_for(nbr_cap, 2 * kChunk, num_sms * (blocks_per_sm > 0 && blocks_per_sm < occ ? blocks_per_sm : occ));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kTThreads);
