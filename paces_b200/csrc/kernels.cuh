@@ -83,17 +83,8 @@ __device__ __forceinline__ void diag_row(bool valid, const C& a, const C& y, dou
     }
 }
 
-// Called by all 32 lanes of a warp for group g, whose rows 64 g + lane (valid0: it exists; a0,
-// y0: v_r and (H v)_r) and 64 g + 32 + lane (valid1, a1, y1) this lane holds.
-template <typename C>
-__device__ __forceinline__ void diag_group(double* __restrict__ diag, int64_t g, bool valid0, const C& a0,
-                                           const C& y0, bool valid1, const C& a1, const C& y1) {
-    double n2, er, ei, n2b, erb, eib;
-    diag_row(valid0, a0, y0, n2, er, ei);
-    diag_row(valid1, a1, y1, n2b, erb, eib);
-    n2 = __dadd_rn(n2, n2b);
-    er = __dadd_rn(er, erb);
-    ei = __dadd_rn(ei, eib);
+// Called by all 32 lanes of a warp for group g: the lanes' sums over their two rows, folded.
+__device__ __forceinline__ void diag_fold(double* __restrict__ diag, int64_t g, double n2, double er, double ei) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         n2 = __dadd_rn(n2, __shfl_xor_sync(0xffffffffu, n2, o));
@@ -105,6 +96,17 @@ __device__ __forceinline__ void diag_group(double* __restrict__ diag, int64_t g,
         diag[g * 3 + 1] = er;
         diag[g * 3 + 2] = ei;
     }
+}
+
+// Called by all 32 lanes of a warp for group g, whose rows 64 g + lane (valid0: it exists; a0,
+// y0: v_r and (H v)_r) and 64 g + 32 + lane (valid1, a1, y1) this lane holds.
+template <typename C>
+__device__ __forceinline__ void diag_group(double* __restrict__ diag, int64_t g, bool valid0, const C& a0,
+                                           const C& y0, bool valid1, const C& a1, const C& y1) {
+    double n2, er, ei, n2b, erb, eib;
+    diag_row(valid0, a0, y0, n2, er, ei);
+    diag_row(valid1, a1, y1, n2b, erb, eib);
+    diag_fold(diag, g, __dadd_rn(n2, n2b), __dadd_rn(er, erb), __dadd_rn(ei, eib));
 }
 
 // ---- Lanczos ----------------------------------------------------------------------------
