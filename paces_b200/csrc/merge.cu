@@ -468,49 +468,17 @@ __global__ void __launch_bounds__(256) merge_split_kernel(ModelDev m, const uint
             }
             if (!any) break;
         }
-        int rank = 0;
+        // its place among the block's splitters in merged order: run jj has a splitter every
+        // `stride` elements, so ceil(co / stride) of them lie before co of its elements
+        int dst = s_off[p * kRuns];
 #pragma unroll
         for (int jj = 0; jj < kRuns; ++jj) {
-            const int co = jj == j ? i : a_[jj];
-            ws.split_co[int64_t(s) * kRuns + jj] = co;
-            rank += co;
+            if (jj == j) a_[jj] = i;
+            dst += (a_[jj] + stride - 1) / stride;
         }
-        ws.split_rank[s] = rank;
-    }
-}
-
-__global__ void __launch_bounds__(256) merge_order_kernel(ModelDev m, MergeWs ws) {
-    const int total = ws.counters[0];
-    const int nr = m.L * kRuns;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < total; s += gridDim.x * blockDim.x) {
-        const int r = find_segment(ws.split_off, nr, s);
-        const int p = r / kRuns, j = r % kRuns;
-        const int own = s - ws.split_off[r];
-        const int rank = ws.split_rank[s];
-        int o = own;
-        int a_[kRuns], b_[kRuns], base_[kRuns];
+        if (dst >= s_off[(p + 1) * kRuns]) continue;  // inconsistent ranks: cannot happen for sorted runs
 #pragma unroll
-        for (int jj = 0; jj < kRuns; ++jj) {
-            a_[jj] = base_[jj] = ws.split_off[p * kRuns + jj];
-            b_[jj] = jj == j ? a_[jj] : ws.split_off[p * kRuns + jj + 1];
-        }
-        for (;;) {  // lockstep searches, as in the split kernel
-            bool any = false;
-#pragma unroll
-            for (int jj = 0; jj < kRuns; ++jj) {
-                if (a_[jj] >= b_[jj]) continue;
-                any = true;
-                const int mid = (a_[jj] + b_[jj]) >> 1;
-                if (ws.split_rank[mid] < rank) a_[jj] = mid + 1; else b_[jj] = mid;
-            }
-            if (!any) break;
-        }
-#pragma unroll
-        for (int jj = 0; jj < kRuns; ++jj) o += a_[jj] - base_[jj];
-        const int64_t dst = int64_t(ws.split_off[p * kRuns]) + o;
-        if (dst >= ws.split_off[(p + 1) * kRuns]) continue;  // inconsistent ranks: cannot happen for sorted runs
-#pragma unroll
-        for (int jj = 0; jj < kRuns; ++jj) ws.ord_co[dst * kRuns + jj] = ws.split_co[int64_t(s) * kRuns + jj];
+        for (int jj = 0; jj < kRuns; ++jj) ws.ord_co[int64_t(dst) * kRuns + jj] = a_[jj];
     }
 }
 
@@ -586,85 +554,102 @@ __device__ long long lookback_warp(unsigned long long* state, int t, long long c
     return excl;
 }
 
-// Everything a tile needs before it loads its elements: its block, segments and merged
-// predecessor (the largest element before the start of any run).  Computed for all tiles at
-// once by merge_desc_kernel, read by the tile kernel with one coalesced load.
+// Everything a tile needs before it merges: its block, segments and merged predecessor (the
+// largest element before the start of any run).
 template <int NW>
 struct TileDesc {
     int p, tl, n, has_pred, pred_flag, nsp;
     int start[kRuns], off[kRuns + 1], lo[kRuns];
-    int pad2;
     uint64_t pred[NW];
     // the merge frontier at the tile's splitters k = 0 .. nsp-1 and at its end (k = nsp): how
     // many elements of each run's segment precede it (every sub-merge of the tile passes
     // through these points)
     uint16_t sc[kMergeGroup + 1][kRuns];
 };
-static_assert(sizeof(TileDesc<kMaxKeyWords>) <= merge_desc_bytes(), "tile descriptor size");
 
-template <int NW>
-__global__ void __launch_bounds__(256) merge_desc_kernel(ModelDev m, const uint64_t* __restrict__ X,
-                                                         const uint64_t* __restrict__ Y, MergeWs ws, int tmax,
-                                                         int* status) {
-    const int ntiles = ws.counters[1];
-    const int L = m.L;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
-        TileDesc<NW> d;
-        const int p = find_segment(ws.tile_off, L, t);
-        const int tl = t - __ldg(ws.tile_off + p);
-        const int ob = __ldg(ws.split_off + p * kRuns);
-        const int nsb = __ldg(ws.split_off + (p + 1) * kRuns) - ob;
-        const int a = ob + tl * kMergeGroup;
-        const int bidx = tl * kMergeGroup + kMergeGroup;
+// Fill the descriptor of tile t; by all lanes of one warp.  s_toff / s_soff: the first tile and
+// the first splitter of every block.  `issue` runs on lane 0 once the segments are known, before
+// the predecessor's keys are read.
+template <int NW, class F>
+__device__ __forceinline__ void tile_setup(const ModelDev& m, const uint64_t* __restrict__ X,
+                                           const uint64_t* __restrict__ Y, const MergeWs& ws, const int* s_toff,
+                                           const int* s_soff, int t, int tmax, TileDesc<NW>& d, int* status, F issue) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;  // blocks that start at or before tile t
+    for (int q = lane; q - lane < m.L; q += 32) before += __popc(__ballot_sync(0xffffffffu, q < m.L && s_toff[q] <= t));
+    const int p = before - 1;
+    const int tl = t - s_toff[p];
+    const int ob = s_soff[p], nsb = s_soff[p + 1] - ob;
+    const int first = tl * kMergeGroup, nsp = min(kMergeGroup, nsb - first);
+    constexpr int kPts = (kMergeGroup + 1) * kRuns, kPer = (kPts + 31) / 32;
+    auto point = [&](int e) -> int {  // co-rank of run e % kRuns at frontier point e / kRuns
+        if (e / kRuns < nsp || first + kMergeGroup < nsb) return __ldcg(ws.ord_co + int64_t(ob + first) * kRuns + e);
+        return __ldcg(ws.run_len + p * kRuns + e % kRuns);  // the end (and unused points)
+    };
+    int co[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) co[q] = q * 32 + lane < kPts ? point(q * 32 + lane) : 0;
+    const int end = lane < kRuns ? point(kPts - kRuns + lane) : 0;
+    const int lo = lane < kRuns ? __ldcg(ws.run_lo + p * kRuns + lane) : 0;
+    const int start = lane < kRuns ? co[0] : 0;  // run j's is point j
+    const int len = max(end - start, 0);
+    int incl = lane < kRuns ? len : 0;  // prefix over the five runs
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, kRuns - 1);
+    // more than a tile holds cannot happen for sorted runs (see merge_tmax); flag it, emit nothing
+    const bool ok = total <= tmax;
+    if (!ok && lane == 0) raise_status(status, PACES_ERR_CAPACITY);
+    if (lane < kRuns) {
+        d.lo[lane] = lo;
+        d.start[lane] = start;
+        d.off[lane] = ok ? incl - len : 0;
+    }
+    if (lane == 0) {
         d.p = p;
         d.tl = tl;
-        d.pad2 = 0;
-        const int nsp = min(kMergeGroup, nsb - tl * kMergeGroup);
+        d.n = d.off[kRuns] = ok ? total : 0;
         d.nsp = nsp;
-        int n = 0, has = 0, pf = 0;
-        Key<NW> pk;
+    }
+    __syncwarp();
+    if (lane == 0) issue();
 #pragma unroll
-        for (int q = 0; q < NW; ++q) pk.w[q] = 0;
-        for (int j = 0; j < kRuns; ++j) {
-            const int st = __ldcg(ws.ord_co + int64_t(a) * kRuns + j);
-            const int en = bidx < nsb ? __ldcg(ws.ord_co + int64_t(ob + bidx) * kRuns + j)
-                                      : __ldg(ws.run_len + p * kRuns + j);
-            const int lo = __ldg(ws.run_lo + p * kRuns + j);
-            d.start[j] = st;
-            d.lo[j] = lo;
-            d.off[j] = n;
-            n += en - st;
-            for (int k = 0; k <= kMergeGroup; ++k) {
-                int c = en - st;  // the end (and unused points)
-                if (k < nsp) c = __ldcg(ws.ord_co + int64_t(a + k) * kRuns + j) - st;
-                d.sc[k][j] = uint16_t(min(max(c, 0), en - st));
-            }
-            if (st > 0) {
-                Key<NW> k;
-                int f;
-                run_elem<NW>(m, X, Y, ws, p, j, int64_t(lo) + st - 1, k, f);
-                // a later run wins ties: it sorts after the earlier one
-                if (!has || cmp_kf(k, f, pk, pf) >= 0) {
-                    pk = k;
-                    pf = f;
-                    has = 1;
-                }
-            }
+    for (int q = 0; q < kPer; ++q) {
+        const int e = q * 32 + lane, j = e % kRuns;
+        const int st = __shfl_sync(0xffffffffu, start, j), ln = __shfl_sync(0xffffffffu, len, j);
+        if (e < kPts) d.sc[e / kRuns][j] = uint16_t(min(max(co[q] - st, 0), ln));
+    }
+    Key<NW> mine;
+    int minef = 0;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) mine.w[q] = 0;
+    const bool has = lane < kRuns && ok && start > 0;
+    if (has) run_elem<NW>(m, X, Y, ws, p, lane, int64_t(lo) + start - 1, mine, minef);
+    const unsigned any = __ballot_sync(0xffffffffu, has);
+    Key<NW> pk = mine;
+    int pf = minef;
+    bool got = any & 1u;  // run 0's, broadcast below
+#pragma unroll
+    for (int j = 0; j < kRuns; ++j) {
+        Key<NW> k;
+#pragma unroll
+        for (int q = 0; q < NW; ++q) k.w[q] = __shfl_sync(0xffffffffu, mine.w[q], j);
+        const int f = __shfl_sync(0xffffffffu, minef, j);
+        // a later run wins ties: it sorts after the earlier one
+        if (j == 0 || (((any >> j) & 1u) && (!got || cmp_kf(k, f, pk, pf) >= 0))) {
+            pk = k;
+            pf = f;
+            got |= (any >> j) & 1u;
         }
-        d.off[kRuns] = n;
-        d.n = n;
-        if (n > tmax) {
-            // cannot happen for sorted runs (see merge_tmax); flag it and emit nothing
-            raise_status(status, PACES_ERR_CAPACITY);
-            for (int j = 0; j <= kRuns; ++j) d.off[j] = 0;
-            d.n = 0;
-            has = 0;
-        }
-        d.has_pred = has;
+    }
+    if (lane == 0) {
+        d.has_pred = got ? 1 : 0;
         d.pred_flag = pf;
 #pragma unroll
         for (int q = 0; q < NW; ++q) d.pred[q] = pk.w[q];
-        *reinterpret_cast<TileDesc<NW>*>(ws.tile_desc + size_t(t) * merge_desc_bytes()) = d;
     }
 }
 
@@ -702,6 +687,19 @@ __device__ void merge_finalize(const ModelDev& m, const MergeWs& ws, const Merge
     if (ceiling_out) *ceiling_out = (ceiling_add ? *ceiling_out : 0) + __ldcg(ws.counters + 3);
 }
 
+// Dynamic shared memory of a tile block: keys, order flags, then uint16 arrays -- merged order,
+// two merge levels (the first becomes the running counts) and, for the split expansion, the new
+// part's running counts -- then the blocks' first tiles and splitters.
+template <int NW>
+__host__ __device__ constexpr size_t tile_blocks_offset(int tmax, int mode) {
+    return (size_t(tmax) * sizeof(Key<NW>) + size_t((tmax + 15) & ~15) +
+            size_t(tmax) * (mode == MERGE_EXPAND_SPLIT ? 8 : 6) + 3) & ~size_t(3);
+}
+template <int NW>
+size_t tile_smem_bytes(int tmax, int mode, int L) {
+    return tile_blocks_offset<NW>(tmax, mode) + size_t(2) * (L + 1) * sizeof(int);
+}
+
 template <int NW, int MODE>
 __global__ void __launch_bounds__(kTileThreads)
 merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __restrict__ Y, MergeWs ws,
@@ -719,13 +717,16 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
     uint16_t* s_cntn = s_lv2 + tmax;   // split only: the same for the new part
     __shared__ int s_t;
     __shared__ long long s_base;
-    __shared__ int s_thr[kTileThreads], s_thrn[kTileThreads];  // exclusive count before each thread
+    __shared__ uint16_t s_thr[kTileThreads], s_thrn[kTileThreads];  // exclusive count before each thread
     __shared__ int s_warp[kTileThreads / 32], s_warpn[kTileThreads / 32];
     __shared__ int s_ceil;
     __shared__ __align__(16) TileDesc<NW> s_d;
     __shared__ uint32_t s_ft[kSubMerges][kFrontiers];
     __shared__ __align__(8) uint64_t s_mbar;  // completion of the tile's bulk copies
     __shared__ int s_abort;
+    // first tile and first splitter of every block (behind the uint16 arrays)
+    int* s_toff = reinterpret_cast<int*>(smem + tile_blocks_offset<NW>(tmax, MODE));
+    int* s_soff = s_toff + m.L + 1;
     const int* s_start = s_d.start;
     const int* s_off = s_d.off;
     const int* s_lo = s_d.lo;
@@ -733,8 +734,10 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
     const int tid = threadIdx.x;
     const int lane = tid & 31, wid = tid >> 5;
     const int ntiles = ws.counters[1];
-    constexpr int kDescWords = int(sizeof(TileDesc<NW>) / 4);
-
+    for (int q = tid; q <= m.L; q += kTileThreads) {
+        s_toff[q] = __ldcg(ws.tile_off + q);
+        s_soff[q] = __ldcg(ws.split_off + q * kRuns);
+    }
     // tiles are taken by ticket when a block starts them (the order the decoupled look-back
     // waits in): the next ticket is drawn at the end of each tile, before its last barrier
     if (tid == 0) {
@@ -748,10 +751,25 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
     for (;;) {
         const int t = s_t;
         if (t >= ntiles) break;
-        // tile set-up: the precomputed descriptor
-        if (tid < kDescWords)
-            reinterpret_cast<int*>(&s_d)[tid] =
-                __ldcg(reinterpret_cast<const int*>(ws.tile_desc + size_t(t) * merge_desc_bytes()) + tid);
+        // 1. the tile's segments into shared memory.  Keys of 16-byte multiples: one bulk copy per
+        //    run segment (completion on the mbarrier, bounded wait)
+        if (wid == 0) {
+            tile_setup<NW>(m, X, Y, ws, s_toff, s_soff, t, tmax, s_d, status, [&]() {
+                if constexpr (NW % 2 == 0) {
+                    const uint32_t mb = tc::smem_addr(&s_mbar);
+                    if (s_d.n <= 0) return;
+                    // the block's reads of the previous tile's keys precede the copies' writes
+                    tc::fence_proxy_async();
+                    tc::mbar_expect_tx(mb, uint32_t(s_d.n) * uint32_t(NW * 8));
+                    for (int j = 0; j < kRuns; ++j) {
+                        const int len = s_off[j + 1] - s_off[j];
+                        if (len <= 0) continue;
+                        const uint64_t* src = (j == RUN_SELF ? X : Y) + (int64_t(s_lo[j]) + s_start[j]) * NW;
+                        tc::bulk_g2s(tc::smem_addr(s_key.w + size_t(s_off[j]) * NW), src, uint32_t(len) * (NW * 8), mb);
+                    }
+                }
+            });
+        }
         __syncthreads();
         const int n = min(s_d.n, tmax);
         const int p = s_d.p;
@@ -760,22 +778,9 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
 #pragma unroll
         for (int q = 0; q < NW; ++q) s_pred.w[q] = s_d.pred[q];
 
-        // 1. the tile's segments into shared memory, transforms applied
+        // transforms applied in place
         if constexpr (NW % 2 == 0) {
-            // keys of 16-byte multiples: one bulk copy per run segment (completion on the
-            // mbarrier, bounded wait), then the transforms in place
             const uint32_t mb = tc::smem_addr(&s_mbar);
-            if (tid == 0 && n > 0) {
-                // the block's reads of the previous tile's keys precede the copies' writes
-                tc::fence_proxy_async();
-                tc::mbar_expect_tx(mb, uint32_t(n) * uint32_t(NW * 8));
-                for (int j = 0; j < kRuns; ++j) {
-                    const int len = s_off[j + 1] - s_off[j];
-                    if (len <= 0) continue;
-                    const uint64_t* src = (j == RUN_SELF ? X : Y) + (int64_t(s_lo[j]) + s_start[j]) * NW;
-                    tc::bulk_g2s(tc::smem_addr(s_key.w + size_t(s_off[j]) * NW), src, uint32_t(len) * (NW * 8), mb);
-                }
-            }
             if (n > 0) {
                 if (!tc::mbar_wait(mb, parity) && lane == 0) s_abort = 1;
                 parity ^= 1u;
@@ -866,8 +871,8 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
             s_warp[wid] = incl;
             s_warpn[wid] = incln;
         }
-        s_thr[tid] = incl - cnt;  // exclusive inside the warp; the warp's offset is added below
-        s_thrn[tid] = incln - cntn;
+        s_thr[tid] = uint16_t(incl - cnt);  // exclusive inside the warp; the warp's offset is added below
+        s_thrn[tid] = uint16_t(incln - cntn);
         __syncthreads();
         if (wid == 0) {
             int v = lane < kTileThreads / 32 ? s_warp[lane] : 0;
@@ -1039,18 +1044,10 @@ __global__ void __launch_bounds__(256) nbr_fill_kernel(ModelDev m, const int* __
     }
 }
 
-template <int NW>
-size_t tile_smem_bytes(int tmax, int mode) {
-    // keys, order flags, then uint16 arrays: merged order, two merge levels (the first becomes
-    // the running counts) and, for the split expansion, the new part's running counts
-    return size_t(tmax) * sizeof(Key<NW>) + size_t((tmax + 15) & ~15) +
-           size_t(tmax) * (mode == MERGE_EXPAND_SPLIT ? 8 : 6);
-}
-
 template <int NW, int MODE>
 void launch_tile(int tmax, const ModelDev& m, const uint64_t* X, const uint64_t* Y, const MergeWs& ws,
                  const MergeOut& out, int* ceiling_out, int ceiling_add, int* status, int num_sms, cudaStream_t st) {
-    const size_t smem = tile_smem_bytes<NW>(tmax, MODE);
+    const size_t smem = tile_smem_bytes<NW>(tmax, MODE, m.L);
     auto kfn = merge_tile_kernel<NW, MODE>;
     cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     int per_sm = 0;
@@ -1078,8 +1075,6 @@ int launch_merge_t(int mode, int stride, const ModelDev& m, const uint64_t* X, c
     if (mode == MERGE_ASSEMBLE && !split_input && out.nbr) o.self_rows_filled = 1;  // nbr_fill_kernel below
     const int g = grid_for(ws.split_cap, 256, num_sms * 8);
     merge_split_kernel<NW><<<g, 256, 0, st>>>(m, X, Y, x_blk, y_blk, ws, stride, status);
-    merge_order_kernel<<<g, 256, 0, st>>>(m, ws);
-    merge_desc_kernel<NW><<<grid_for(ws.tile_cap, 256, num_sms * 8), 256, 0, st>>>(m, X, Y, ws, tmax, status);
     if (mode == MERGE_ASSEMBLE)
         launch_tile<NW, MERGE_ASSEMBLE>(tmax, m, X, Y, ws, o, ceiling_out, ceiling_add, status, num_sms, st);
     else if (mode == MERGE_EXPAND_SPLIT)

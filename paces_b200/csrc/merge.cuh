@@ -41,11 +41,8 @@ struct MergeWs {
     int* tile_off;   // [L + 1] prefix of tile counts
     int* counters;   // [0] splitters [1] tiles [2] tile ticket [3] ceiling holes [4] output count
                      // [5] tile blocks done
-    int* split_co;   // [split_cap * kRuns]
-    int* split_rank; // [split_cap]
-    int* ord_co;     // [split_cap * kRuns]
+    int* ord_co;     // [split_cap * kRuns] co-ranks of the splitters, each block's in merged order
     unsigned long long* tile_state;  // [tile_cap] look-back words
-    unsigned char* tile_desc;        // [tile_cap] tile descriptors (merge_desc_bytes each)
     int split_cap;
     int tile_cap;
     // optional candidate filter (expansion only): keep[j * keep_cap + src] == 0 drops the
@@ -148,8 +145,6 @@ inline int64_t merge_split_cap(int64_t in_cap, int nw, int L) {
     return kRuns * (in_cap / kMinMergeStride + 1) + int64_t(kRuns) * L + 8;
 }
 inline int64_t merge_tile_cap(int64_t split_cap, int L) { return split_cap / kMergeGroup + L + 8; }
-// Bytes of one tile descriptor (any key width).
-constexpr size_t merge_desc_bytes() { return 320; }
 
 // X feeds the self run, Y (null: X) the four image runs.  ceiling_out (optional) receives the
 // number of ceiling holes of the up run, or has it added (ceiling_add).  An assembly with
