@@ -91,29 +91,59 @@ obs_energy_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict
 
 // `uniform`: every field is `ub` bits wide and word q holds sites q*fpw .. q*fpw+fpw-1
 // MSB-first (NW <= 4), so thread-private register accumulators cover all sites.  UB = 4
-// (the width for occupation cut-offs up to 15) masks each field in place at a constant
-// position; UB = 0 reads the width from `ub`.  A field value becomes a double exactly by
+// (the width for occupation cut-offs up to 15) and UB = 2 (up to 3, NW <= 2) mask each field in
+// place at a constant position; UB = 0 reads the width from `ub` (>= 4).  UB = -1 is every
+// other layout.  A field value becomes a double exactly by
 // the 2^52 offset (its bits under the exponent of 2^52, minus 2^52): two FP64-pipe
 // operations instead of an integer conversion, whose pipe is a quarter as wide.
 template <int NW, bool C64, int UB>
-__global__ void __launch_bounds__(kOThreads, NW <= 2 ? 2 : 1)
+__global__ void __launch_bounds__(kOThreads, UB < 0 ? 3 : (NW * (UB == 2 ? 32 : kFpwMax) <= 32 ? 2 : 1))
 obs_sites_kernel(ModelDev m, const uint64_t* __restrict__ keys, const int* __restrict__ blk,
                  const uint32_t* __restrict__ meta, const void* __restrict__ psi, double* __restrict__ part,
-                 int uniform_in, int ub, int fpw) {
+                 int ub, int fpw) {
     using C = typename std::conditional<C64, float2, double2>::type;
-    constexpr bool kFast = NW <= 4;
-    constexpr int kAcc = kFast ? NW * kFpwMax : 1;
+    constexpr bool uniform = UB >= 0;
+    constexpr int kFpw = UB == 2 ? 32 : kFpwMax;
+    constexpr int kAcc = uniform ? NW * kFpw : 1;
+    // UB > 0: the bit of a field's least significant bit in its 32-bit half
+    auto low_bit = [](int f) { return 32 - UB - UB * (f % (UB > 0 ? 32 / UB : 1)); };
     __shared__ double s_site[kOWarps][2 * kMaxSites];
     __shared__ double s_red[kOWarps];
     const int L = m.L;
     const int nv = 1 + 2 * L;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const bool uniform = kFast && uniform_in;
     const uint64_t umask = (uint64_t(1) << ub) - 1;
     double racc[kAcc];
 #pragma unroll
     for (int i = 0; i < kAcc; ++i) racc[i] = 0.0;
-    double pho[4] = {0.0, 0.0, 0.0, 0.0}, exc[4] = {0.0, 0.0, 0.0, 0.0};
+    double pho[4] = {0.0, 0.0, 0.0, 0.0};
+    struct Rows {
+        uint64_t key[32][NW];
+        double w[32];
+    };
+    __shared__ Rows s_rows[uniform ? 1 : kOWarps];  // general layouts
+    int sw[4], ssh[4];
+    uint32_t smk[4];
+#pragma unroll
+    for (int qi = 0; qi < 4; ++qi) {
+        const int s = min(lane + 32 * qi, L - 1);
+        sw[qi] = m.word[s];
+        ssh[qi] = m.shift[s];
+        smk[qi] = lane + 32 * qi < L ? (1u << m.bits[s]) - 1u : 0u;
+    }
+    auto walk_rows = [&](auto groups) {
+        constexpr int G = decltype(groups)::value;
+        const auto& rows = s_rows[uniform ? 0 : wid];
+#pragma unroll 4
+        for (int i = 0; i < 32; ++i) {
+            const double ws = rows.w[i];
+#pragma unroll
+            for (int qi = 0; qi < G; ++qi) {
+                const uint32_t nf = uint32_t(rows.key[i][sw[qi]] >> ssh[qi]) & smk[qi];
+                pho[qi] = fma(ws, __hiloint2double(0x43300000, int(nf)) - 4503599627370496.0, pho[qi]);
+            }
+        }
+    };
     for (int k = threadIdx.x; k < kOWarps * 2 * kMaxSites; k += kOThreads) (&s_site[0][0])[k] = 0.0;
     __syncthreads();
     const int64_t S = blk[L];
@@ -167,7 +197,7 @@ obs_sites_kernel(ModelDev m, const uint64_t* __restrict__ keys, const int* __res
             for (int q = 0; q < NW; ++q) k.w[q] = 0;
         }
         norm2 += w;
-        if (uniform) {
+        {
             // n_exc: the warp's rows lie in one exciton block or straddle a few; while they stay
             // in the block of the previous rows, each lane keeps adding to its own sum
             const int pme = int(mm & 0xffu);
@@ -190,61 +220,56 @@ obs_sites_kernel(ModelDev m, const uint64_t* __restrict__ keys, const int* __res
                     }
                 }
             }
+        }
+        if constexpr (uniform) {
             if (valid && w != 0.0) {
 #pragma unroll
                 for (int q = 0; q < NW; ++q) {
                     const uint64_t word = k.w[q];
                     const uint32_t whi = uint32_t(word >> 32), wlo = uint32_t(word);
 #pragma unroll
-                    for (int f = 0; f < kFpwMax; ++f) {
-                        if (UB == 4 || f < fpw) {
-                            // UB = 4: the field left in place, n * 2^(28 - 4 (f mod 8)) of its
-                            // 32-bit half (one AND); the sum is scaled back at the end
+                    for (int f = 0; f < kFpw; ++f) {
+                        if (UB > 0 || f < fpw) {
+                            // UB > 0: the field left in place, n * 2^low_bit(f) of its 32-bit half
+                            // (one AND); the sum is scaled back at the end
                             uint32_t nf;
-                            if constexpr (UB == 4) nf = (f < 8 ? whi : wlo) & (15u << (28 - 4 * (f & 7)));
+                            if constexpr (UB > 0) nf = (f < kFpw / 2 ? whi : wlo) & (((1u << UB) - 1u) << low_bit(f));
                             else nf = uint32_t((word >> (64 - ub * (f + 1))) & umask);
                             const double dn = __hiloint2double(0x43300000, int(nf)) - 4503599627370496.0;
-                            racc[q * kFpwMax + f] = fma(w, dn, racc[q * kFpwMax + f]);
+                            racc[q * kFpw + f] = fma(w, dn, racc[q * kFpw + f]);
                         }
                     }
                 }
             }
         } else {
-            // general layout: broadcast each row; lane l owns sites l, l+32, l+64, l+96
-            unsigned act = __ballot_sync(0xffffffffu, valid && w != 0.0);
-            while (act) {
-                const int src = __ffs(act) - 1;
-                act &= act - 1;
-                const double ws = __shfl_sync(0xffffffffu, w, src);
-                const int ps = __shfl_sync(0xffffffffu, int(mm & 0xffu), src);
-                Key<NW> kk;
+            // general layout: lane l owns sites l, l+32, l+64, l+96 and walks the 32 rows, their
+            // keys and weights in shared memory (a row's word is one broadcast load; with the row
+            // passed by shuffles and its fields looked up per row this pass took 315 us for 866K
+            // rows of 16 sites)
 #pragma unroll
-                for (int q = 0; q < NW; ++q) kk.w[q] = __shfl_sync(0xffffffffu, k.w[q], src);
-#pragma unroll
-                for (int qi = 0; qi < 4; ++qi) {
-                    const int s = lane + 32 * qi;
-                    if (s < L) {
-                        pho[qi] += ws * double(get_field(m, kk, s));
-                        if (ps == s) exc[qi] += ws;
-                    }
-                }
-            }
+            for (int q = 0; q < NW; ++q) s_rows[wid].key[lane][q] = k.w[q];
+            s_rows[wid].w[lane] = w;  // 0 past the last row
+            __syncwarp();
+            if (L <= 32) walk_rows(std::integral_constant<int, 1>{});
+            else if (L <= 64) walk_rows(std::integral_constant<int, 2>{});
+            else walk_rows(std::integral_constant<int, 4>{});
+            __syncwarp();
         }
     }
     flush_exc();
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) norm2 += __shfl_xor_sync(0xffffffffu, norm2, o);
     if (lane == 0) s_red[wid] = norm2;
-    if (uniform) {
+    if constexpr (uniform) {
 #pragma unroll
         for (int i = 0; i < kAcc; ++i) {
-            // UB = 4 sums carry the field's position 2^(28 - 4 (f mod 8)): every product and
-            // partial sum is exactly that power of two times the unscaled one (no overflow or
-            // underflow at these magnitudes), so the scaled-back sum has the same bits
-            double v = UB == 4 ? racc[i] * (1.0 / double(1u << (28 - 4 * ((i % kFpwMax) & 7)))) : racc[i];
+            // UB > 0: the sums carry the field's position 2^low_bit: every product and partial sum
+            // is exactly that power of two times the unscaled one (no overflow or underflow at
+            // these magnitudes), so the scaled-back sum has the same bits
+            double v = UB > 0 ? racc[i] * (1.0 / double(1u << low_bit(i % kFpw))) : racc[i];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            const int q = i / kFpwMax, f = i % kFpwMax;
+            const int q = i / kFpw, f = i % kFpw;
             const int s = q * fpw + f;
             if (lane == 0 && f < fpw && s < L) s_site[wid][L + s] = v;
         }
@@ -252,10 +277,7 @@ obs_sites_kernel(ModelDev m, const uint64_t* __restrict__ keys, const int* __res
 #pragma unroll
         for (int qi = 0; qi < 4; ++qi) {
             const int s = lane + 32 * qi;
-            if (s < L) {
-                s_site[wid][s] = exc[qi];
-                s_site[wid][L + s] = pho[qi];
-            }
+            if (s < L) s_site[wid][L + s] = pho[qi];
         }
     }
     __syncthreads();
@@ -572,12 +594,14 @@ template <int NW, bool C64>
 int launch_obs_t(const ModelDev& m, const uint64_t* keys, const int* blk, const int* nbr,
                  int64_t nbr_cap, const uint32_t* meta, const void* psi, int what, double* partials,
                  const ObsTarget& out, int num_sms, cudaStream_t st) {
-    static int grid_e = 0, grid_ex = 0, grid_s = 0, grid_s4 = 0;
+    static int grid_e = 0, grid_ex = 0, grid_s = 0, grid_s4 = 0, grid_s2 = 0, grid_sg = 0;
     if (grid_e == 0) {
         grid_e = wave_blocks(obs_energy_kernel<C64, false>, num_sms);
         grid_ex = wave_blocks(obs_energy_kernel<C64, true>, num_sms);
-        grid_s = wave_blocks(obs_sites_kernel<NW, C64, 0>, num_sms);
+        grid_sg = wave_blocks(obs_sites_kernel<NW, C64, -1>, num_sms);
+        if constexpr (NW <= 4) grid_s = wave_blocks(obs_sites_kernel<NW, C64, 0>, num_sms);
         if constexpr (NW <= 4) grid_s4 = wave_blocks(obs_sites_kernel<NW, C64, 4>, num_sms);
+        if constexpr (NW <= 2) grid_s2 = wave_blocks(obs_sites_kernel<NW, C64, 2>, num_sms);
     }
     const bool energy = (what & PACES_OBS_ENERGY) != 0;
     const bool sites = (what & PACES_OBS_SITES) != 0;
@@ -596,21 +620,35 @@ int launch_obs_t(const ModelDev& m, const uint64_t* keys, const int* blk, const 
     if (sites) {
         int ub = m.bits[0];
         const int fpw = ub > 0 ? 64 / ub : 0;
-        bool uniform = ub >= 4 && NW <= 4;
+        // narrow fields: 2-bit ones have their own instance, the others take the general walk
+        bool uniform = (ub >= 4 && NW <= 4) || (ub == 2 && NW <= 2);
         for (int s = 0; s < m.L && uniform; ++s)
             uniform = m.bits[s] == ub && m.word[s] == s / fpw && m.shift[s] == 64 - ub * (s % fpw + 1);
         bool done = false;
         if constexpr (NW <= 4) {
             if (uniform && ub == 4) {
-                obs_sites_kernel<NW, C64, 4><<<grid_s4, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, 1, ub, fpw);
+                obs_sites_kernel<NW, C64, 4><<<grid_s4, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
                 nb_s = grid_s4;
                 done = true;
             }
         }
+        if constexpr (NW <= 2) {
+            if (uniform && ub == 2) {
+                obs_sites_kernel<NW, C64, 2><<<grid_s2, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
+                nb_s = grid_s2;
+                done = true;
+            }
+        }
+        if constexpr (NW <= 4) {
+            if (uniform && !done) {
+                obs_sites_kernel<NW, C64, 0><<<grid_s, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
+                nb_s = grid_s;
+                done = true;
+            }
+        }
         if (!done) {
-            obs_sites_kernel<NW, C64, 0><<<grid_s, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s,
-                                                                      uniform ? 1 : 0, ub, fpw);
-            nb_s = grid_s;
+            obs_sites_kernel<NW, C64, -1><<<grid_sg, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
+            nb_s = grid_sg;
         }
     }
     obs_final_kernel<<<sites ? 3 + 2 * m.L : 3, 256, 0, st>>>(m.L, nb_e, part_e, nb_s, part_s, out);
