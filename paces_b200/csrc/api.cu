@@ -83,8 +83,7 @@ struct Layout {
     size_t keysA, blkA, keysB, blkB, maps;
     size_t m_run_lo, m_run_len, m_split_off, m_tile_off, m_counters, m_ord_co, m_tile_state;
     int64_t split_cap, tile_cap;
-    size_t t_hist, t_cand, t_cand_idx, t_sel, t_tile_cnt, t_tile_pre;
-    int t_tiles;
+    size_t t_hist, t_cand, t_cand_idx, t_sel, t_sum, t_chunk;
     size_t r_tile_off, r_counters, r_split;
     int r_tiles;
     size_t v_V, v_TA, v_TB, v_partials, v_bar;
@@ -121,13 +120,12 @@ Layout make_layout(const paces_ctx* c, int64_t cap) {
     l.m_counters = take(16 * 4);
     l.m_ord_co = take(size_t(l.split_cap) * kRuns * 4);
     l.m_tile_state = take(size_t(l.tile_cap) * 8);
-    l.t_tiles = trunc_tiles_cap(cap);
-    l.t_hist = take(4096 * 4);
+    l.t_hist = take(kTruncHistBytes);
     l.t_cand = take(ucap * 8);
     l.t_cand_idx = take(ucap * 4);
     l.t_sel = take(16 * 8);
-    l.t_tile_cnt = take(size_t(l.t_tiles) * 3 * 4);
-    l.t_tile_pre = take(size_t(l.t_tiles) * 3 * 4);
+    l.t_sum = take(1024 * 8);
+    l.t_chunk = take(size_t(trunc_chunks_cap(cap)) * 8);
     l.r_tiles = remap_tile_cap(cap, nw, L);
     l.r_tile_off = take(size_t(L + 1) * 4);
     l.r_counters = take(16);
@@ -198,10 +196,10 @@ TruncWs trunc_ws(const Layout& l, void* ws) {
     w.cand = at<unsigned long long>(ws, l.t_cand);
     w.cand_idx = at<int>(ws, l.t_cand_idx);
     w.sel = at<long long>(ws, l.t_sel);
-    w.tile_cnt = at<int>(ws, l.t_tile_cnt);
-    w.tile_pre = at<int>(ws, l.t_tile_pre);
+    w.barrier = w.hist + 3 * 4096;
+    w.block_sum = at<unsigned long long>(ws, l.t_sum);
+    w.chunk = at<unsigned long long>(ws, l.t_chunk);
     w.cap = l.cap;
-    w.ntiles_cap = l.t_tiles;
     return w;
 }
 
@@ -425,16 +423,15 @@ int plan_step(paces_ctx* c, const paces_basis* old_b, const void* old_psi, paces
 // Kernels one step enqueues (merge: 2 per pass, +1 for the neighbour table; truncation: see
 // trunc_launches, +1 with look-ahead weights; remap 2; observables 2 or 3; Taylor 1;
 // renormalisation 3; record 2).
-unsigned long long step_launches(const paces_step_params& prm, bool c64, bool with_taylor, int passes) {
-    const int wk = prm.weighting ? 2 : (c64 ? 1 : 0);
-    return 2 + (prm.weighting ? 1 : 0) + trunc_launches(wk, prm.shuffle != 0) +
+unsigned long long step_launches(const paces_step_params& prm, bool with_taylor, int passes) {
+    return 2 + (prm.weighting ? 1 : 0) + trunc_launches(prm.shuffle != 0) +
            (prm.proposal && prm.enlarge_steps > 0 ? 1 : 0) + 2ull * passes * (prm.enlarge_steps + 1) + 1 +
            2 + (prm.diagnostics ? 2 : 0) +
            (prm.evolve ? (with_taylor ? 1 : 0) + (prm.renormalize ? 3 : 0) : 0) + 3;
 }
 
 // Record, truncation, enlargement, new basis + H, remap, post-adaptation diagnostics.
-int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks) {
+int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks, int at_once = 1) {
     const bool c64 = c->precision == PACES_C64;
     const paces_step_params* prm = p.prm;
     paces_step_record* rec = p.rec;
@@ -461,7 +458,8 @@ int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks) {
     PACES_CHECK_LAUNCH(c, launch_truncate(c->nw, c64, c->m, p.old_b->keys, p.old_b->blk, p.old_psi, weights, wscratch,
                                           prm->maxstates,
                                           prm->shuffle, prm->shuffle_seed, prm->step_index, trunc_ws(l, ws), p.A.keys,
-                                          p.A.blk, p.A.cap, at<float>(ws, l.aw), &rec->n_tied, &rec->n_select, status, c->num_sms, st),
+                                          p.A.blk, p.A.cap, at<float>(ws, l.aw), &rec->n_tied, &rec->n_select, status, c->num_sms, at_once,
+                                          st),
                        "step/truncate");
     // 1b. learned proposal: score the truncated basis' images
     const bool propose = prm->proposal && prm->enlarge_steps > 0;
@@ -979,7 +977,7 @@ int paces_truncate(paces_ctx* c, const paces_basis* in, const void* psi, int64_t
     if (in->cap > l.cap) return fail(c, PACES_ERR_CAPACITY, "workspace holds %lld states, input basis %lld", (long long)l.cap, (long long)in->cap);
     PACES_CHECK_LAUNCH(c, launch_truncate(c->nw, c->precision == PACES_C64, c->m, in->keys, in->blk, psi, nullptr,
                                           at<void>(ws, l.v_TA), maxstates, shuffle, shuffle_seed, step_index, trunc_ws(l, ws), out->keys,
-                                          out->blk, out->cap, nullptr, nullptr, nullptr, c->d_status, c->num_sms,
+                                          out->blk, out->cap, nullptr, nullptr, nullptr, c->d_status, c->num_sms, 1,
                                           reinterpret_cast<cudaStream_t>(stream)),
                        "truncate");
     return PACES_OK;
@@ -993,7 +991,7 @@ int paces_truncate_weighted(paces_ctx* c, const paces_basis* in, const double* w
     if (in->cap > l.cap) return fail(c, PACES_ERR_CAPACITY, "workspace holds %lld states, input basis %lld", (long long)l.cap, (long long)in->cap);
     PACES_CHECK_LAUNCH(c, launch_truncate(c->nw, c->precision == PACES_C64, c->m, in->keys, in->blk, nullptr, weights,
                                           nullptr, maxstates, shuffle, shuffle_seed, step_index, trunc_ws(l, ws), out->keys,
-                                          out->blk, out->cap, nullptr, nullptr, nullptr, c->d_status, c->num_sms,
+                                          out->blk, out->cap, nullptr, nullptr, nullptr, c->d_status, c->num_sms, 1,
                                           reinterpret_cast<cudaStream_t>(stream)),
                        "truncate_weighted");
     return PACES_OK;
@@ -1214,7 +1212,7 @@ int paces_step(paces_ctx* c, const paces_basis* old_b, const void* old_psi, pace
     const int rc = plan_step(c, old_b, old_psi, new_b, new_psi, h, prm, rec, ws, ws_bytes, &p);
     if (rc != PACES_OK) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    c->launches += step_launches(*prm, c->precision == PACES_C64, true, merge_passes(c->m));
+    c->launches += step_launches(*prm, true, merge_passes(c->m));
     int r = step_front(c, p, st, true);
     if (r != PACES_OK) return r;
     if (prm->evolve) {
@@ -1423,7 +1421,7 @@ int paces_batch_step(paces_batch* b, const paces_batch_item* items, int32_t n, p
         const int rc = plan_step(it.ctx, it.old_basis, it.old_psi, it.new_basis, it.new_psi, it.h, it.params,
                                  it.record, it.workspace, it.workspace_bytes, &plans[i]);
         if (rc != PACES_OK) return bfail(rc, "item %d: %s", i, it.ctx->err);
-        launches += step_launches(*it.params, it.ctx->precision == PACES_C64, false, merge_passes(it.ctx->m));
+        launches += step_launches(*it.params, false, merge_passes(it.ctx->m));
         n_evolve += it.params->evolve ? 1 : 0;
     }
     auto fork = [&]() -> bool {
@@ -1447,7 +1445,7 @@ int paces_batch_step(paces_batch* b, const paces_batch_item* items, int32_t n, p
     mark(0);
     if (!fork()) return bfail(PACES_ERR_CUDA, "fork: %s", cudaGetErrorString(cudaGetLastError()));
     for (int i = 0; i < n; ++i) {
-        const int rc = step_front(items[i].ctx, plans[i], b->streams[i % b->n_streams], false);
+        const int rc = step_front(items[i].ctx, plans[i], b->streams[i % b->n_streams], false, b->n_streams);
         if (rc != PACES_OK) {
             join();
             return bfail(rc, "item %d: %s", i, items[i].ctx->err);

@@ -1,6 +1,7 @@
 // Amplitude-ranked truncation (see truncate.cuh).
 #include <type_traits>
 
+#include "grid.cuh"
 #include "truncate.cuh"
 
 namespace paces {
@@ -68,24 +69,9 @@ __device__ __forceinline__ unsigned long long tie_hash(uint64_t seed, uint64_t s
     return ~z;  // keep the largest ~hash == the smallest hash
 }
 
-__global__ void trunc_init_kernel(ModelDev m, const int* __restrict__ x_blk, int64_t maxstates,
-                                  TruncWs ws) {
-    const int tid = threadIdx.x;
-    for (int b = tid; b < 4096; b += blockDim.x) ws.hist[b] = 0;
-    if (tid == 0) {
-        const long long S = x_blk[m.L];
-        for (int k = 0; k < SEL_WORDS; ++k) ws.sel[k] = 0;
-        ws.sel[SEL_S] = S;
-        ws.sel[SEL_ALL] = S <= maxstates ? 1 : 0;
-        ws.sel[SEL_W + 2] = maxstates;
-        ws.sel[SEL_W + 3] = S <= maxstates ? 0 : 1;
-    }
-}
-
-// One radix round: find the digit holding the need-th largest key, narrow the prefix;
-// on the final round (record_ties) the chosen bin's count is the number of tied states.
-__global__ void __launch_bounds__(1024) trunc_select_kernel(TruncWs ws, int base, int round,
-                                                            int record_ties) {
+// One radix round of the tie shuffle: find the digit holding the need-th largest hash and
+// narrow the prefix.
+__global__ void __launch_bounds__(1024) trunc_select_kernel(TruncWs ws, int base, int round) {
     __shared__ long long s_warp[32];
     __shared__ int s_bin;
     __shared__ long long s_above;
@@ -133,64 +119,300 @@ __global__ void __launch_bounds__(1024) trunc_select_kernel(TruncWs ws, int base
         ws.sel[base + 2] = need - s_above;
         ws.sel[base + 0] |= (long long)((unsigned long long)b << shift);
         ws.sel[base + 1] |= (long long)((unsigned long long)(nb - 1) << shift);
-        if (record_ties) ws.sel[SEL_TIES] = ws.hist[b];
     }
     __syncthreads();
     for (int b = tid; b < 4096; b += blockDim.x) ws.hist[b] = 0;
 }
 
-// One radix round over all states: histogram of the round's digit among the states whose
-// higher digits equal the prefix chosen so far (round 0: every state).  A full streaming
-// pass per round -- no candidate list, so no global counter and no scattered writes.  Lanes
-// with the same digit add to the shared histogram once (warp-aggregated: in round 0 most
-// states share a few binades).
-// STORE (round 0 of |psi| kinds): also write every state's weight to `wout` in the stored
-// kind, which the later passes read instead of recomputing |psi|.
-template <int WK, bool STORE>
-__global__ void __launch_bounds__(256) trunc_hist_pass_kernel(const void* __restrict__ psi, TruncWs ws, int round,
-                                                              void* __restrict__ wout, int* status) {
-    __shared__ unsigned h[4096];
-    if (!ws.sel[SEL_W + 3]) return;
-    const int bits = round_bits(round), shift = round_shift(round);
-    const unsigned long long dm = (1ull << bits) - 1;
-    for (int b = threadIdx.x; b < (1 << bits); b += blockDim.x) h[b] = 0;
-    __syncthreads();
-    const int64_t S = ws.sel[SEL_S];
-    const unsigned long long pre = (unsigned long long)ws.sel[SEL_W + 0];
-    const unsigned long long msk = (unsigned long long)ws.sel[SEL_W + 1];
+constexpr int kSelThreads = 1024;
+constexpr int kSelWarps = kSelThreads / 32;
+constexpr int kU = kTruncChunk / 32;  // states per lane of a chunk, their loads in flight together
+constexpr int kSelCand = 2048;        // a bin this small is settled from a list of its weights
+// the first pass's bins: 2^-63 .. 2 in steps of 2^-6 of a binade
+constexpr int kFirstShift = 46;
+constexpr unsigned long long kFirstBase = (unsigned long long)(1023 - 63) << 52;
+
+// Calls f(chunk, weight bits, existing states' bits) for chunks [c0, c1) of kTruncChunk states,
+// `warps` warps of which this is number w: lane l holds states 32 u + l of the chunk.
+template <int K, class F>
+__device__ __forceinline__ void for_chunks(const void* from, int64_t S, int64_t c0, int64_t c1, int w, int warps,
+                                           int* status, F f) {
     const int lane = threadIdx.x & 31;
-    // warp chunks of 4 x 32 states: the four loads of a lane are in flight together
-    constexpr int kU = 4;
-    const int64_t nwarps = int64_t(gridDim.x) * (blockDim.x >> 5);
-    for (int64_t c = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); c * 32 * kU < S; c += nwarps) {
-        RawW<WK> z[kU];
+    for (int64_t c = c0 + w; c < c1; c += warps) {
+        const int64_t i0 = c * kTruncChunk + lane;
+        constexpr int kG = sizeof(RawW<K>) >= 16 ? kU / 2 : kU;  // loads in flight together
+        unsigned ok = 0;
+        unsigned long long k[kU];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int64_t i = (c * kU + u) * 32 + lane;
-            if (i < S) z[u] = load_raw<WK>(psi, i);
-        }
+        for (int g = 0; g < kU; g += kG) {
+            RawW<K> z[kG];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int64_t i = (c * kU + u) * 32 + lane;
-            bool match = false;
-            unsigned bin = 0xffffffffu;
-            if (i < S) {
-                const unsigned long long k = raw_bits<WK>(z[u], status);
-                if constexpr (STORE) {
-                    const double wv = __longlong_as_double((long long)k);
-                    if constexpr (stored_kind(WK) == 3) reinterpret_cast<float*>(wout)[i] = float(wv);
-                    else reinterpret_cast<double*>(wout)[i] = wv;
+            for (int u = 0; u < kG; ++u) {
+                if (i0 + 32 * (g + u) < S) {
+                    z[u] = load_raw<K>(from, i0 + 32 * (g + u));
+                    ok |= 1u << (g + u);
                 }
-                match = (k & msk) == pre;
-                if (match) bin = unsigned((k >> shift) & dm);
             }
-            const unsigned peers = __match_any_sync(0xffffffffu, bin);
-            if (match && lane == __ffs(peers) - 1) atomicAdd(&h[bin], unsigned(__popc(peers)));
+#pragma unroll
+            for (int u = 0; u < kG; ++u) k[g + u] = ok >> (g + u) & 1u ? raw_bits<K>(z[u], status) : 0ull;
+        }
+        f(c, k, ok);
+    }
+}
+
+// Block-wide exclusive prefix of one value per thread; `total` gets the block's sum.  s_sum:
+// one word per warp.
+__device__ unsigned long long block_prefix(unsigned long long v, unsigned long long* s_sum, unsigned long long& total) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned long long incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+    }
+    __syncthreads();
+    if (lane == 31) s_sum[wid] = incl;
+    __syncthreads();
+    unsigned long long before = 0;
+    total = 0;
+    for (int w = 0; w < int(blockDim.x >> 5); ++w) {
+        const unsigned long long x = s_sum[w];
+        if (w < wid) before += x;
+        total += x;
+    }
+    return before + incl - v;
+}
+
+// The need-th largest of a histogram's entries, by all threads of the block: thread t holds the
+// counts hb[] of bins [t * PER, (t + 1) * PER).  s_pick: bin, entries above it, its count.
+template <int PER>
+__device__ __forceinline__ void pick_bin(const unsigned (&hb)[PER], long long need, long long* s_warp, long long* s_pick) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    long long mine = 0;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) mine += hb[q];
+    long long incl = mine;  // this thread's bins and those of the higher lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long v = __shfl_down_sync(0xffffffffu, incl, o);
+        if (lane + o < 32) incl += v;
+    }
+    if (lane == 0) s_warp[wid] = incl;
+    if (tid == 0) s_pick[0] = -1;
+    __syncthreads();
+    long long above = incl - mine;
+    for (int w = wid + 1; w < int(blockDim.x >> 5); ++w) above += s_warp[w];
+    if (mine > 0 && above < need && need <= above + mine) {
+#pragma unroll
+        for (int q = PER - 1; q >= 0; --q) {
+            if (above < need && need <= above + hb[q]) {
+                s_pick[0] = tid * PER + q;
+                s_pick[1] = above;
+                s_pick[2] = hb[q];
+            }
+            above += hb[q];
         }
     }
     __syncthreads();
-    for (int b = threadIdx.x; b < (1 << bits); b += blockDim.x)
-        if (h[b]) atomicAdd(&ws.hist[b], h[b]);
+}
+
+// The selection in one cooperative launch, one block of 1024 threads per SM.
+//  * The threshold's bits lie in [lo, lo + width): streaming passes, each into a shared-memory
+//    histogram of 4096 bins over that range, a grid barrier, and every block picking the bin
+//    from the grid's histogram itself.  The first pass bins 64 binades below 2 by 6 mantissa
+//    bits (what lies below or above goes to its end bins): exponents alone put most states
+//    into a few bins, whose atomics collide.
+//  * Once the chosen bin holds at most kSelCand states (two passes leave a few of millions;
+//    all bits take up to 6 passes), one more pass lists the bin's states and every block
+//    settles the remaining bits among them.
+//  * That pass also counts the states above the bin per chunk of the compaction; with the
+//    listed states added and the blocks' totals exchanged, the counts become every chunk's
+//    prefix (states above the threshold | tied states << 31), so the compaction's warps need
+//    nothing from each other.
+// A launch per pass and selection, and a counting and a scanning launch, took 85 us for 15K
+// complex128 states, nearly all of it latency.
+//
+// STORE: the first round computes |psi| and writes it to `wout` in the stored kind, which the
+// later passes read (each thread its own states).
+template <int WK, bool STORE>
+__global__ void __launch_bounds__(kSelThreads, 1)
+trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restrict__ psi, TruncWs ws,
+                       int64_t maxstates, void* wout, int low, int* status) {
+    constexpr int WS = STORE ? stored_kind(WK) : WK;  // the kind the passes after the first read
+    __shared__ unsigned h[4096];
+    __shared__ long long s_warp[kSelWarps], s_pick[3];
+    __shared__ unsigned long long s_sum[kSelWarps], s_own;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int64_t S = x_blk[L];
+    const bool all = S <= maxstates;
+    if (blockIdx.x == 0 && tid < SEL_WORDS) {
+        // until the selection is known: nothing to write (a wait that runs out leaves it so)
+        long long v = 0;
+        if (tid == SEL_ALL) v = 1;
+        if (all && tid == SEL_S) v = S;
+        ws.sel[tid] = v;
+    }
+    if (all) return;
+    const int64_t nch = (S + kTruncChunk - 1) / kTruncChunk;
+    const int64_t c0 = nch * blockIdx.x / gridDim.x, c1 = nch * (blockIdx.x + 1) / gridDim.x;  // this block's chunks
+    unsigned gen = 0;
+    unsigned long long lo = 0, width = ~0ull;
+    long long need = maxstates, count = S;
+    const void* src = psi;
+    // width - 1 takes this many bits; bits below `low` are zero in every weight
+    auto bits_of = [](unsigned long long x) { return 64 - __clzll((long long)(x - 1)); };
+    for (int round = 0;; ++round) {
+        const int shift = round == 0 ? kFirstShift : max(bits_of(width) - 12, 0);
+        for (int b = tid; b < 4096; b += kSelThreads) h[b] = 0;
+        __syncthreads();
+        if (round == 0) {
+            for_chunks<WK>(src, S, c0, c1, wid, kSelWarps, status, [&](int64_t c, const unsigned long long (&k)[kU], unsigned ok) {
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    if (!(ok >> u & 1u)) continue;
+                    if constexpr (STORE) {
+                        const double wv = __longlong_as_double((long long)k[u]);
+                        const int64_t i = c * kTruncChunk + 32 * u + lane;
+                        if constexpr (WS == 3) reinterpret_cast<float*>(wout)[i] = float(wv);
+                        else reinterpret_cast<double*>(wout)[i] = wv;
+                    }
+                    const long long b = (long long)(k[u] >> kFirstShift) - (long long)(kFirstBase >> kFirstShift);
+                    atomicAdd(&h[int(min(max(b, 0ll), 4095ll))], 1u);
+                }
+            });
+            if constexpr (STORE) src = wout;
+        } else {
+            for_chunks<WS>(src, S, c0, c1, wid, kSelWarps, status, [&](int64_t, const unsigned long long (&k)[kU], unsigned ok) {
+#pragma unroll
+                for (int u = 0; u < kU; ++u)
+                    if ((ok >> u & 1u) && k[u] - lo < width) atomicAdd(&h[unsigned((k[u] - lo) >> shift)], 1u);
+            });
+        }
+        __syncthreads();
+        unsigned* gh = ws.hist + (round % 3) * 4096;
+        for (int b = tid; b < 4096; b += kSelThreads)
+            if (h[b]) atomicAdd(&gh[b], h[b]);
+        if (!grid_barrier(ws.barrier, gridDim.x, gen, status)) return;
+        constexpr int per = 4096 / kSelThreads;
+        unsigned hb[per];
+#pragma unroll
+        for (int q = 0; q < per; ++q) hb[q] = __ldcg(gh + tid * per + q);
+        if (blockIdx.x == 0)  // the histogram of the round after next
+            for (int b = tid; b < 4096; b += kSelThreads) ws.hist[((round + 2) % 3) * 4096 + b] = 0;
+        pick_bin<per>(hb, need, s_warp, s_pick);
+        if (s_pick[0] < 0) {  // cannot happen: the states' count does not change between rounds
+            if (blockIdx.x == 0 && tid == 0) raise_status(status, PACES_ERR_BADARG);
+            return;
+        }
+        const unsigned long long bin = (unsigned long long)s_pick[0];
+        if (round > 0) {
+            lo += bin << shift;
+            width = 1ull << shift;
+        } else {
+            lo = bin == 0 ? 0ull : kFirstBase + (bin << shift);
+            width = bin == 0 ? kFirstBase + (1ull << shift) : (bin == 4095 ? 0ull - lo : 1ull << shift);
+        }
+        need -= s_pick[1];
+        count = s_pick[2];
+        if (width <= (1ull << low) || count <= kSelCand) break;
+        __syncthreads();  // s_pick has been read
+    }
+    // the chunks' counts; the bin's states listed, or (every bit decided) counted as the tied ones
+    const bool list = width > (1ull << low);
+    if (tid == 0) s_own = 0;
+    __syncthreads();
+    for_chunks<WS>(src, S, c0, c1, wid, kSelWarps, status, [&](int64_t c, const unsigned long long (&k)[kU], unsigned ok) {
+        unsigned na = 0, nt = 0;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const bool v = (ok >> u & 1u) && k[u] >= lo, in = v && k[u] - lo < width;
+            na += __popc(__ballot_sync(0xffffffffu, v && !in));
+            if (list) {
+                if (in) {
+                    const unsigned slot = atomicAdd(ws.barrier + 1, 1u);
+                    if (slot < kSelCand && slot < ws.cap) {
+                        ws.cand[slot] = k[u];
+                        ws.cand_idx[slot] = int(c * kTruncChunk + 32 * u + lane);
+                    }
+                }
+            } else {
+                nt += __popc(__ballot_sync(0xffffffffu, in));
+            }
+        }
+        if (lane == 0) {
+            const unsigned long long n = (unsigned long long)na | ((unsigned long long)nt << 31);
+            ws.chunk[c] = n;
+            atomicAdd(&s_own, n);
+        }
+    });
+    long long ties = count;
+    if (list) {
+        if (!grid_barrier(ws.barrier, gridDim.x, gen, status)) return;
+        // the need-th largest of the listed weights, 12 bits a round
+        const int n = int(count);
+        constexpr int kMine = kSelCand / kSelThreads, per = 4096 / kSelThreads;
+        unsigned long long w[kMine];
+        int wi[kMine];
+#pragma unroll
+        for (int q = 0; q < kMine; ++q) {
+            const int i = tid + q * kSelThreads;
+            const bool have = i < n && i < ws.cap;
+            w[q] = have ? __ldcg(ws.cand + i) : 0ull;
+            wi[q] = have ? __ldcg(ws.cand_idx + i) : -1;
+        }
+        while (width > (1ull << low)) {
+            const int shift = max(bits_of(width) - 12, 0);
+            __syncthreads();
+            for (int b = tid; b < 4096; b += kSelThreads) h[b] = 0;
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < kMine; ++q)
+                if (wi[q] >= 0 && w[q] - lo < width) atomicAdd(&h[unsigned((w[q] - lo) >> shift)], 1u);
+            __syncthreads();
+            unsigned hb[per];
+#pragma unroll
+            for (int q = 0; q < per; ++q) hb[q] = h[tid * per + q];
+            pick_bin<per>(hb, need, s_warp, s_pick);
+            if (s_pick[0] < 0) {  // cannot happen, as above
+                if (blockIdx.x == 0 && tid == 0) raise_status(status, PACES_ERR_BADARG);
+                return;
+            }
+            lo += (unsigned long long)s_pick[0] << shift;
+            width = 1ull << shift;
+            need -= s_pick[1];
+            ties = s_pick[2];
+        }
+        // this block's listed states join its chunks' counts
+#pragma unroll
+        for (int q = 0; q < kMine; ++q) {
+            const int64_t c = wi[q] / kTruncChunk;
+            if (wi[q] < 0 || c < c0 || c >= c1 || w[q] < lo) continue;
+            const unsigned long long one = w[q] - lo >= width ? 1ull : 1ull << 31;
+            atomicAdd(ws.chunk + c, one);
+            atomicAdd(&s_own, one);
+        }
+    }
+    // exclusive prefixes: the blocks' totals, then this block's chunks
+    __syncthreads();
+    if (tid == 0) ws.block_sum[blockIdx.x] = s_own;
+    if (!grid_barrier(ws.barrier, gridDim.x, gen, status)) return;
+    unsigned long long before, total;
+    block_prefix(tid < blockIdx.x ? __ldcg(ws.block_sum + tid) : 0ull, s_sum, before);
+    for (int64_t c = c0; c < c1; c += kSelThreads) {
+        const unsigned long long v = c + tid < c1 ? __ldcg(ws.chunk + c + tid) : 0ull;
+        const unsigned long long e = block_prefix(v, s_sum, total);
+        if (c + tid < c1) ws.chunk[c + tid] = before + e;
+        before += total;
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        ws.sel[SEL_W + 0] = (long long)lo;
+        ws.sel[SEL_W + 1] = -1;  // every bit decided
+        ws.sel[SEL_W + 2] = need;
+        ws.sel[SEL_W + 3] = 1;
+        ws.sel[SEL_TIES] = ties;
+        ws.sel[SEL_S] = S;
+        ws.sel[SEL_ALL] = 0;
+    }
 }
 
 __global__ void __launch_bounds__(256) trunc_hist_cand_kernel(TruncWs ws, int base, int round) {
@@ -213,7 +435,8 @@ __global__ void __launch_bounds__(256) trunc_hist_cand_kernel(TruncWs ws, int ba
 }
 
 // Decide whether the tie at the cut is shuffled; if so, collect the tied states' hashes.
-__global__ void trunc_shuffle_prep_kernel(TruncWs ws, int* status) {
+__global__ void __launch_bounds__(1024) trunc_shuffle_prep_kernel(TruncWs ws, int* status) {
+    for (int b = threadIdx.x; b < 4096; b += blockDim.x) ws.hist[b] = 0;
     if (threadIdx.x != 0) return;
     const long long ties = ws.sel[SEL_TIES];
     const long long need = ws.sel[SEL_W + 2];
@@ -254,271 +477,149 @@ __global__ void __launch_bounds__(256) trunc_collect_ties_kernel(const void* __r
     }
 }
 
-// Per tile: states above the threshold, tied states, tied states kept by the hash rule.
+// With shuffled ties: the chunks' kept states (above the threshold, or tied and picked by the
+// hash), then their prefixes.
 template <int WK>
-__global__ void __launch_bounds__(256) trunc_count_kernel(const void* __restrict__ psi, TruncWs ws,
-                                                          uint64_t seed, uint64_t step, int* status) {
-    __shared__ int s_c[3];
+__global__ void __launch_bounds__(256) trunc_shuffle_count_kernel(const void* __restrict__ psi, TruncWs ws, uint64_t seed,
+                                                                  uint64_t step, int* status) {
+    if (ws.sel[SEL_ALL] || !ws.sel[SEL_SHUFFLE]) return;
     const int64_t S = ws.sel[SEL_S];
-    const int ntiles = int((S + kTruncTile - 1) / kTruncTile);
-    if (ws.sel[SEL_ALL]) return;
     const unsigned long long vstar = (unsigned long long)ws.sel[SEL_W + 0];
-    const bool shuf = ws.sel[SEL_SHUFFLE] != 0;
     const unsigned long long hstar = (unsigned long long)ws.sel[SEL_H + 0];
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        if (threadIdx.x < 3) s_c[threadIdx.x] = 0;
-        __syncthreads();
-        int a = 0, ti = 0, hk = 0;
-        const int64_t i1 = min(S, int64_t(t + 1) * kTruncTile);
-        constexpr int kU = 4;  // loads in flight per thread
-        for (int64_t i0 = int64_t(t) * kTruncTile + threadIdx.x; i0 < i1; i0 += kU * int64_t(blockDim.x)) {
-            RawW<WK> z[kU];
+    const int lane = threadIdx.x & 31;
+    for_chunks<WK>(psi, S, 0, (S + kTruncChunk - 1) / kTruncChunk, int(blockIdx.x * 8 + (threadIdx.x >> 5)), int(gridDim.x * 8),
+                   status, [&](int64_t c, const unsigned long long (&k)[kU], unsigned ok) {
+                       unsigned n = 0;
 #pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (i0 + u * int64_t(blockDim.x) < i1) z[u] = load_raw<WK>(psi, i0 + u * int64_t(blockDim.x));
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int64_t i = i0 + u * int64_t(blockDim.x);
-                if (i >= i1) break;
-                const unsigned long long k = raw_bits<WK>(z[u], status);
-                a += k > vstar;
-                if (k == vstar) {
-                    ++ti;
-                    if (shuf) hk += tie_hash(seed, step, i) >= hstar;
-                }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            ti += __shfl_xor_sync(0xffffffffu, ti, o);
-            hk += __shfl_xor_sync(0xffffffffu, hk, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&s_c[0], a);
-            atomicAdd(&s_c[1], ti);
-            atomicAdd(&s_c[2], hk);
-        }
-        __syncthreads();
-        if (threadIdx.x < 3) ws.tile_cnt[t * 3 + threadIdx.x] = s_c[threadIdx.x];
-        __syncthreads();
+                       for (int u = 0; u < kU; ++u) {
+                           const bool keep = (ok >> u & 1u) &&
+                                             (k[u] > vstar || (k[u] == vstar &&
+                                                               tie_hash(seed, step, c * kTruncChunk + 32 * u + lane) >= hstar));
+                           n += __popc(__ballot_sync(0xffffffffu, keep));
+                       }
+                       if (lane == 0) ws.chunk[c] = n;
+                   });
+}
+
+__global__ void __launch_bounds__(1024) trunc_shuffle_scan_kernel(TruncWs ws) {
+    __shared__ unsigned long long s_sum[32];
+    if (ws.sel[SEL_ALL] || !ws.sel[SEL_SHUFFLE]) return;
+    const int64_t nch = (ws.sel[SEL_S] + kTruncChunk - 1) / kTruncChunk;
+    unsigned long long before = 0, total;
+    for (int64_t c = threadIdx.x; c - threadIdx.x < nch; c += blockDim.x) {
+        const unsigned long long e = block_prefix(c < nch ? ws.chunk[c] : 0ull, s_sum, total);
+        if (c < nch) ws.chunk[c] = before + e;
+        before += total;
     }
 }
 
-__global__ void __launch_bounds__(1024) trunc_scan_kernel(TruncWs ws) {
-    __shared__ int s_w[32][3];
-    if (ws.sel[SEL_ALL]) return;
-    const int64_t S = ws.sel[SEL_S];
-    const int ntiles = int((S + kTruncTile - 1) / kTruncTile);
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int per = (ntiles + 1023) / 1024;
-    const int t0 = min(tid * per, ntiles), t1 = min(t0 + per, ntiles);
-    int c[3] = {0, 0, 0};
-    for (int t = t0; t < t1; ++t)
-        for (int k = 0; k < 3; ++k) c[k] += ws.tile_cnt[t * 3 + k];
-    int incl[3];
-    for (int k = 0; k < 3; ++k) {
-        incl[k] = c[k];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl[k], o);
-            if (lane >= o) incl[k] += v;
-        }
-        if (lane == 31) s_w[wid][k] = incl[k];
-    }
-    __syncthreads();
-    if (tid < 3) {
-        int acc = 0;
-        for (int w = 0; w < 32; ++w) {
-            const int v = s_w[w][tid];
-            s_w[w][tid] = acc;
-            acc += v;
-        }
-    }
-    __syncthreads();
-    int run[3];
-    for (int k = 0; k < 3; ++k) run[k] = s_w[wid][k] + incl[k] - c[k];
-    for (int t = t0; t < t1; ++t)
-        for (int k = 0; k < 3; ++k) {
-            ws.tile_pre[t * 3 + k] = run[k];
-            run[k] += ws.tile_cnt[t * 3 + k];
-        }
-}
-
-// The compaction: every warp owns kTruncTile / 8 consecutive states of the tile.  Pass 1
-// counts, per warp, the states above the threshold, the tied ones and the tied ones the
-// hash keeps (ballots); pass 2 walks the same states 32 at a time and places every kept
-// state at its rank among the kept ones (ballot prefixes).  Lanes read consecutive keys
-// and the kept ones write consecutive outputs, so both sides coalesce.
+// The compaction: a warp holds the weights of a chunk's 256 consecutive states in registers,
+// ballots and the chunk's prefix give every kept state its rank among the kept ones.  Lanes
+// read consecutive keys and the kept ones write consecutive outputs, so both sides coalesce,
+// and no warp waits for another (a look-back over 1024-state tiles in place of the prefixes:
+// 158 us at 15.2M states).
 // The weights come from `wsrc` (kind WK); when every state is kept the selection rounds
-// did not run, so the out_w weights come from `psi` (kind WKA).
+// did not run, so the out_w weights come from `psi` (kind WKA).  The last block to finish
+// writes the offsets of empty exciton blocks and the counts.
 template <int NW, int WK, int WKA>
-__global__ void __launch_bounds__(256) trunc_write_kernel(ModelDev m, const uint64_t* __restrict__ x_keys,
+__global__ void __launch_bounds__(256, NW <= 2 ? 4 : (NW <= 4 ? 3 : 2)) trunc_write_kernel(ModelDev m, const uint64_t* __restrict__ x_keys,
                                                           const int* __restrict__ x_blk,
                                                           const void* __restrict__ wsrc,
-                                                          const void* __restrict__ psi, TruncWs ws,
+                                                          const void* __restrict__ psi, TruncWs ws, int64_t maxstates,
                                                           uint64_t seed, uint64_t step,
                                                           uint64_t* __restrict__ out_keys,
                                                           int* __restrict__ out_blk, int64_t out_cap,
-                                                          float* __restrict__ out_w, int* status) {
-    constexpr int kWarps = 8;
-    constexpr int kSeg = kTruncTile / kWarps;
-    __shared__ unsigned long long s_k[kTruncTile];
+                                                          float* __restrict__ out_w, int* n_tied_out, int* n_kept_out,
+                                                          int* status) {
     __shared__ int s_blk[kMaxSites + 1];
-    __shared__ int s_w[kWarps][3];
     const int L = m.L;
     for (int i = threadIdx.x; i <= L; i += blockDim.x) s_blk[i] = x_blk[i];
+    __syncthreads();
     const int64_t S = ws.sel[SEL_S];
     const bool all = ws.sel[SEL_ALL] != 0;
-    const int ntiles = int((S + kTruncTile - 1) / kTruncTile);
     const unsigned long long vstar = (unsigned long long)ws.sel[SEL_W + 0];
-    const long long need = ws.sel[SEL_W + 2];
-    const long long ties = ws.sel[SEL_TIES];
-    const long long skip_ties = ties - need;  // tied states dropped (the lowest indices)
+    const long long skip_ties = ws.sel[SEL_TIES] - ws.sel[SEL_W + 2];  // tied states dropped (the lowest indices)
     const bool shuf = ws.sel[SEL_SHUFFLE] != 0;
     const unsigned long long hstar = (unsigned long long)ws.sel[SEL_H + 0];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
-    __syncthreads();
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int64_t i0 = int64_t(t) * kTruncTile;
-        const int n = int(min(int64_t(kTruncTile), S - i0));
-        const int q_lo = min(wid * kSeg, n), q_hi = min(q_lo + kSeg, n);
-        // pass 1: weights into shared memory, per-warp counts
-        int ca = 0, ct = 0, ch = 0;
-        if (!all || out_w) {
-            constexpr int kU = 4;  // loads in flight per lane
-            if (WK != WKA && all) {
-                // every state kept (early steps only): out_w from the amplitudes
-                for (int q = q_lo + lane; q < q_hi; q += 32) s_k[q] = raw_bits<WKA>(load_raw<WKA>(psi, i0 + q), status);
+    auto place = [&](int64_t c, const unsigned long long (&k)[kU], unsigned ok) {
+        const int64_t q0 = c * kTruncChunk;
+        const unsigned long long b = all ? (unsigned long long)q0 : __ldg(ws.chunk + c);
+        long long T = (long long)(b >> 31);  // tied states before the chunk
+        long long out = (long long)(b & 0x7fffffffull);
+        if (!all && !shuf) out += max(0ll, T - skip_ties);
+        const long long out0 = out;
+        unsigned kept[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const bool v = ok >> u & 1u;
+            const bool eq = v && !all && k[u] == vstar;
+            bool keep = v && (all || k[u] > vstar);
+            if (shuf) {
+                keep |= eq && tie_hash(seed, step, q0 + 32 * u + lane) >= hstar;
             } else {
-                for (int q0 = q_lo; q0 < q_hi; q0 += 32 * kU) {
-                    RawW<WK> z[kU];
+                const unsigned tie = __ballot_sync(0xffffffffu, eq);
+                keep |= eq && T + __popc(tie & lt_mask) >= skip_ties;
+                T += __popc(tie);
+            }
+            kept[u] = __ballot_sync(0xffffffffu, keep);
+        }
+        constexpr int kG = 4;  // keys in flight per lane
 #pragma unroll
-                    for (int u = 0; u < kU; ++u) {
-                        const int q = q0 + 32 * u + lane;
-                        if (q < q_hi) z[u] = load_raw<WK>(wsrc, i0 + q);
-                    }
+        for (int g = 0; g < kU; g += kG) {
+            Key<NW> kk[kG];
 #pragma unroll
-                    for (int u = 0; u < kU; ++u) {
-                        const int q = q0 + 32 * u + lane;
-                        if (q < q_hi) s_k[q] = raw_bits<WK>(z[u], status);
+            for (int u = 0; u < kG; ++u)
+                if (kept[g + u] >> lane & 1u) kk[u] = load_key<NW>(x_keys, q0 + 32 * (g + u) + lane);
+#pragma unroll
+            for (int u = 0; u < kG; ++u) {
+                if (kept[g + u] >> lane & 1u) {
+                    const long long o = out + __popc(kept[g + u] & lt_mask);
+                    if (o < out_cap) {
+                        store_key<NW>(out_keys, o, kk[u]);
+                        if (out_w) out_w[o] = float(__longlong_as_double((long long)k[g + u]));
+                    } else {
+                        raise_status(status, PACES_ERR_CAPACITY);
                     }
                 }
-            }
-            __syncwarp();
-            if (!all)
-                for (int q0 = q_lo; q0 < q_hi; q0 += 32) {
-                    const int q = q0 + lane;
-                    const bool v = q < q_hi;
-                    const unsigned long long k = v ? s_k[q] : 0ull;
-                    const bool tie = v && k == vstar;
-                    ca += __popc(__ballot_sync(0xffffffffu, v && k > vstar));
-                    ct += __popc(__ballot_sync(0xffffffffu, tie));
-                    if (shuf) ch += __popc(__ballot_sync(0xffffffffu, tie && tie_hash(seed, step, i0 + q) >= hstar));
-                }
-        }
-        if (lane == 0) {
-            s_w[wid][0] = ca;
-            s_w[wid][1] = ct;
-            s_w[wid][2] = ch;
-        }
-        __syncthreads();
-        long long A = 0, T = 0, H = 0;
-        if (!all) {
-            A = ws.tile_pre[t * 3 + 0];
-            T = ws.tile_pre[t * 3 + 1];
-            H = ws.tile_pre[t * 3 + 2];
-            for (int w = 0; w < wid; ++w) {
-                A += s_w[w][0];
-                T += s_w[w][1];
-                H += s_w[w][2];
+                out += __popc(kept[g + u]);
             }
         }
-        // pass 2: ranks among the kept states, block starts, copies; four slices of 32 per
-        // round, their key loads in flight together.  Exciton blocks start in few of the
-        // warp's segments: a warp whose segment holds no block start skips their search.
-        bool starts = false;
+        // exciton blocks that start among the chunk's states: the kept states before them
         for (int p = lane; p < L; p += 32) {
-            const int64_t b0 = s_blk[p];
-            starts |= b0 >= i0 + q_lo && b0 < i0 + q_hi && b0 < s_blk[p + 1];
-        }
-        starts = __any_sync(0xffffffffu, starts);
-        constexpr int kU = 4;
-        for (int qb = q_lo; qb < q_hi; qb += 32 * kU) {
-            bool keep[kU];
-            long long out[kU];
+            const int64_t e = int64_t(s_blk[p]) - q0;
+            if (e < 0 || e >= kTruncChunk || s_blk[p] >= s_blk[p + 1]) continue;
+            long long o = out0;
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
-                const int q0 = qb + 32 * u;
-                const int q = q0 + lane;
-                const bool v = q < q_hi;
-                const int64_t i = i0 + q;
-                if (all) {
-                    keep[u] = v;
-                    out[u] = i;
-                } else {
-                    const unsigned long long k = v ? s_k[q] : 0ull;
-                    const bool above = v && k > vstar;
-                    const bool tie = v && k == vstar;
-                    const bool hk = shuf && tie && tie_hash(seed, step, i) >= hstar;
-                    const unsigned ba = __ballot_sync(0xffffffffu, above);
-                    const unsigned bt = __ballot_sync(0xffffffffu, tie);
-                    const unsigned bh = __ballot_sync(0xffffffffu, hk);
-                    const long long a_l = A + __popc(ba & lt_mask);
-                    const long long t_l = T + __popc(bt & lt_mask);
-                    const long long h_l = H + __popc(bh & lt_mask);
-                    out[u] = a_l + (shuf ? h_l : max(0ll, t_l - skip_ties));
-                    keep[u] = above || (tie && (shuf ? hk : t_l >= skip_ties));
-                    A += __popc(ba);
-                    T += __popc(bt);
-                    H += __popc(bh);
-                }
-                // block starts among these 32 states: the number of kept states before them
-                for (int p0 = 0; starts && p0 < L; p0 += 32) {
-                    const int p = p0 + lane;
-                    const int e = p < L ? int(int64_t(s_blk[p]) - (i0 + q0)) : -1;
-                    const long long o = __shfl_sync(0xffffffffu, out[u], (e >= 0 && e < 32) ? e : 0);
-                    if (p < L && e >= 0 && e < 32 && q0 + e < q_hi && s_blk[p] < s_blk[p + 1]) out_blk[p] = int(o);
-                }
+                if (u < int(e >> 5)) o += __popc(kept[u]);
+                else if (u == int(e >> 5)) o += __popc(kept[u] & ((1u << (e & 31)) - 1u));
             }
-            Key<NW> kk[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u)
-                if (keep[u] && out[u] < out_cap) kk[u] = load_key<NW>(x_keys, i0 + qb + 32 * u + lane);
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                if (!keep[u]) continue;
-                if (out[u] < out_cap) {
-                    store_key<NW>(out_keys, out[u], kk[u]);
-                    if (out_w) out_w[out[u]] = float(__longlong_as_double((long long)s_k[qb + 32 * u + lane]));
-                } else {
-                    raise_status(status, PACES_ERR_CAPACITY);
-                }
-            }
+            out_blk[p] = int(o);
         }
-        __syncthreads();
-    }
-}
-
-__global__ void trunc_finalize_kernel(ModelDev m, const int* __restrict__ x_blk, int64_t maxstates,
-                                      TruncWs ws, int* out_blk, int64_t out_cap, int* n_tied_out, int* n_kept_out,
-                                      float* cut_out, int* status) {
+    };
+    const int64_t nch = (S + kTruncChunk - 1) / kTruncChunk;
+    const int w = int(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)), warps = int(gridDim.x * (blockDim.x >> 5));
+    if (all) for_chunks<WKA>(psi, S, 0, nch, w, warps, status, place);
+    else for_chunks<WK>(wsrc, S, 0, nch, w, warps, status, place);
+    __syncthreads();
     if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(ws.barrier + 2, 1u) != gridDim.x - 1) return;
+    __threadfence();
     // the cut: |psi| of the smallest kept state when states were dropped, else 0
-    if (cut_out) *cut_out = ws.sel[SEL_ALL] ? 0.f : float(__longlong_as_double(ws.sel[SEL_W + 0]));
-    const int L = m.L;
-    const long long S = ws.sel[SEL_S];
-    long long total = ws.sel[SEL_ALL] ? S : maxstates;
+    if (out_w) out_w[out_cap] = all ? 0.f : float(__longlong_as_double((long long)vstar));
+    long long total = all ? S : maxstates;
     if (total > out_cap) {
         raise_status(status, PACES_ERR_CAPACITY);
         total = out_cap;
     }
     if (ws.sel[SEL_CAND] > ws.cap) raise_status(status, PACES_ERR_CAPACITY);
     out_blk[L] = int(total);
-    for (int p = L - 1; p >= 0; --p)
-        if (x_blk[p] == x_blk[p + 1]) out_blk[p] = out_blk[p + 1];
-    if (n_tied_out) *n_tied_out = int(ws.sel[SEL_ALL] ? 0 : ws.sel[SEL_TIES]);
+    for (int p = L - 1; p >= 0; --p)  // (no states: every block is empty)
+        if (S == 0 || s_blk[p] == s_blk[p + 1]) out_blk[p] = __ldcg(out_blk + p + 1);
+    if (n_tied_out) *n_tied_out = int(all ? 0 : ws.sel[SEL_TIES]);
     if (n_kept_out) *n_kept_out = int(total);
 }
 
@@ -528,32 +629,38 @@ template <int NW, int WK, int WKS>
 int launch_truncate_t(const ModelDev& m, const uint64_t* x_keys, const int* x_blk, const void* psi, void* scratch,
                       int64_t maxstates, int shuffle, uint64_t seed, uint64_t step, const TruncWs& ws,
                       uint64_t* out_keys, int* out_blk, int64_t out_cap, float* out_w, int* n_tied_out, int* n_kept_out,
-                      int* status, int num_sms, cudaStream_t st) {
+                      int* status, int num_sms, int at_once, cudaStream_t st) {
     constexpr bool kStore = WKS != WK;
     const void* src = kStore ? scratch : psi;
-    const int g = grid_for(ws.cap, 1024, num_sms * 4);          // streaming passes
-    const int gt = grid_for(ws.cap, kTruncTile, num_sms * 4);   // passes over 4096-state tiles
-    const int rounds = weight_rounds(WK);
-    trunc_init_kernel<<<1, 1024, 0, st>>>(m, x_blk, maxstates, ws);
-    for (int r = 0; r < rounds; ++r) {
-        if (r == 0) trunc_hist_pass_kernel<WK, kStore><<<g, 256, 0, st>>>(psi, ws, r, scratch, status);
-        else trunc_hist_pass_kernel<WKS, false><<<g, 256, 0, st>>>(src, ws, r, nullptr, status);
-        trunc_select_kernel<<<1, 1024, 0, st>>>(ws, SEL_W, r, r == rounds - 1);
+    const int g = grid_for(ws.cap, 1024, num_sms * 4);  // streaming passes of the tie shuffle
+    if (cudaMemsetAsync(ws.hist, 0, kTruncHistBytes, st) != cudaSuccess) return PACES_ERR_CUDA;
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid_for(ws.cap, kSelThreads * 2, max(num_sms / at_once, 1)));
+        cfg.blockDim = dim3(kSelThreads);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaLaunchKernelEx(&cfg, trunc_threshold_kernel<WK, kStore>, m.L, x_blk, psi, ws, maxstates, scratch,
+                               weight_low_bit(WK), status) != cudaSuccess)
+            return PACES_ERR_CUDA;
     }
     if (shuffle) {
-        trunc_shuffle_prep_kernel<<<1, 32, 0, st>>>(ws, status);
+        trunc_shuffle_prep_kernel<<<1, 1024, 0, st>>>(ws, status);
         trunc_collect_ties_kernel<WKS><<<g, 256, 0, st>>>(src, ws, seed, step, status);
         for (int r = 0; r < kRounds; ++r) {
             trunc_hist_cand_kernel<<<g, 256, 0, st>>>(ws, SEL_H, r);
-            trunc_select_kernel<<<1, 1024, 0, st>>>(ws, SEL_H, r, 0);
+            trunc_select_kernel<<<1, 1024, 0, st>>>(ws, SEL_H, r);
         }
+        trunc_shuffle_count_kernel<WKS><<<g, 256, 0, st>>>(src, ws, seed, step, status);
+        trunc_shuffle_scan_kernel<<<1, 1024, 0, st>>>(ws);
     }
-    trunc_count_kernel<WKS><<<gt, 256, 0, st>>>(src, ws, seed, step, status);
-    trunc_scan_kernel<<<1, 1024, 0, st>>>(ws);
-    trunc_write_kernel<NW, WKS, WK><<<gt, 256, 0, st>>>(m, x_keys, x_blk, src, psi, ws, seed, step, out_keys,
-                                                        out_blk, out_cap, out_w, status);
-    trunc_finalize_kernel<<<1, 32, 0, st>>>(m, x_blk, maxstates, ws, out_blk, out_cap, n_tied_out, n_kept_out,
-                                            out_w ? out_w + out_cap : nullptr, status);
+    trunc_write_kernel<NW, WKS, WK><<<grid_for(ws.cap, 8 * kTruncChunk, num_sms * 8), 256, 0, st>>>(
+        m, x_keys, x_blk, src, psi, ws, maxstates, seed, step, out_keys, out_blk, out_cap, out_w, n_tied_out, n_kept_out,
+        status);
     return cudaGetLastError() == cudaSuccess ? PACES_OK : PACES_ERR_CUDA;
 }
 
@@ -561,11 +668,11 @@ template <int NW>
 int dispatch_prec(bool c64, const ModelDev& m, const uint64_t* x_keys, const int* x_blk,
                   const void* psi, const double* weights, void* scratch, int64_t maxstates, int shuffle, uint64_t seed,
                   uint64_t step, const TruncWs& ws, uint64_t* out_keys, int* out_blk, int64_t out_cap,
-                  float* out_w, int* n_tied_out, int* n_kept_out, int* status, int num_sms, cudaStream_t st) {
+                  float* out_w, int* n_tied_out, int* n_kept_out, int* status, int num_sms, int at_once, cudaStream_t st) {
 #define PACES_TRUNC_LAUNCH(WK, WKS, SRC)                                                                     \
     return launch_truncate_t<NW, WK, WKS>(m, x_keys, x_blk, SRC, scratch, maxstates, shuffle, seed, step, ws, \
                                           out_keys, out_blk, out_cap, out_w, n_tied_out, n_kept_out, status,  \
-                                          num_sms, st)
+                                          num_sms, at_once, st)
     if (weights) PACES_TRUNC_LAUNCH(2, 2, weights);
     if (c64) {
         if (scratch) PACES_TRUNC_LAUNCH(1, stored_kind(1), psi);
@@ -581,11 +688,11 @@ int dispatch_prec(bool c64, const ModelDev& m, const uint64_t* x_keys, const int
 int launch_truncate(int nw, bool c64, const ModelDev& m, const uint64_t* x_keys, const int* x_blk,
                     const void* psi, const double* weights, void* scratch, int64_t maxstates, int shuffle, uint64_t seed,
                     uint64_t step, const TruncWs& ws, uint64_t* out_keys, int* out_blk, int64_t out_cap, float* out_w,
-                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, cudaStream_t st) {
+                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, int at_once, cudaStream_t st) {
 #define PACES_TRUNC_CASE(N)                                                                       \
     case N:                                                                                       \
         return dispatch_prec<N>(c64, m, x_keys, x_blk, psi, weights, scratch, maxstates, shuffle, seed, step, ws, \
-                                out_keys, out_blk, out_cap, out_w, n_tied_out, n_kept_out, status, num_sms, st);
+                                out_keys, out_blk, out_cap, out_w, n_tied_out, n_kept_out, status, num_sms, at_once, st);
     switch (nw) {
         PACES_TRUNC_CASE(1)
         PACES_TRUNC_CASE(2)

@@ -6,7 +6,7 @@
 // cut are drawn at random.
 //
 // B200 design: no sort.  The weights |psi| are non-negative doubles, so their bit
-// patterns order like the values; a radix select (12-bit digits, shared-memory
+// patterns order like the values; a radix select (4096 bins a pass, shared-memory
 // histograms) finds the threshold value v* and the number of states equal to v* that
 // must be kept.  Because the basis is already sorted, keeping the selected states in
 // index order *is* the lexsorted result: one order-preserving compaction writes the
@@ -21,27 +21,26 @@
 namespace paces {
 
 struct TruncWs {
-    unsigned* hist;              // [4096]
+    unsigned* hist;              // [3][4096] radix histograms in rotation
+    unsigned* barrier;           // behind them: grid barrier, listed states, blocks done
     unsigned long long* cand;    // [cap] candidate weight bits (or hashes)
     int* cand_idx;               // [cap]
     long long* sel;              // selection state, see truncate.cu
-    int* tile_cnt;               // [ntiles_cap][3]
-    int* tile_pre;               // [ntiles_cap][3]
+    unsigned long long* block_sum;   // [1024] the selection's blocks: counts of their chunks
+    unsigned long long* chunk;       // [trunc_chunks_cap(cap)] counts, then prefixes of the chunks
     int64_t cap;
-    int ntiles_cap;
 };
+constexpr size_t kTruncHistBytes = (3 * 4096 + 16) * 4;  // histograms and counters, zeroed per truncation
 
-constexpr int kTruncTile = 4096;
+constexpr int kTruncChunk = 256;  // states a warp of the compaction takes at a time
 
-inline int trunc_tiles_cap(int64_t cap) { return int(cap / kTruncTile + 2); }
+inline int64_t trunc_chunks_cap(int64_t cap) { return cap / kTruncChunk + 2; }
 
-// Radix rounds (12-bit digits from the top) of the weight selection for a weight kind (0
-// complex128 |psi|, 1 complex64 |psi|, 2 precomputed fp64 weights): a complex64 weight is
-// an fp32 value widened to a double, so its bits 28..0 are zero and rounds 0-2 (bits
-// 63..28) decide it.
-inline int weight_rounds(int wk) { return wk == 1 ? 3 : 6; }
+// Bits below this one are zero in every weight of a kind (0 complex128 |psi|, 1 complex64
+// |psi|, 2 precomputed fp64 weights): a complex64 weight is an fp32 value widened to a double.
+inline int weight_low_bit(int wk) { return wk == 1 ? 29 : 0; }
 // Kernels one truncation enqueues.
-inline int trunc_launches(int wk, bool shuffle) { return 5 + 2 * weight_rounds(wk) + (shuffle ? 14 : 0); }
+inline int trunc_launches(bool shuffle) { return 2 + (shuffle ? 16 : 0); }
 
 // weights (optional, one non-negative double per state): rank by these instead of |psi|
 // (the look-ahead weighting, lookahead.cu).
@@ -51,9 +50,11 @@ inline int trunc_launches(int wk, bool shuffle) { return 5 + 2 * weight_rounds(w
 // out_w (optional, out_cap + 1 floats): the ranked weight (|psi|) of every kept state in the
 // new basis' order, and at out_w[out_cap] the cut -- the weight of the smallest kept state, 0
 // when nothing was dropped.
+// at_once: truncations that may run at the same time on this GPU; each takes its share of the
+// SMs for the launch whose blocks wait for one another, so all of them fit together.
 int launch_truncate(int nw, bool c64, const ModelDev& m, const uint64_t* x_keys, const int* x_blk,
                     const void* psi, const double* weights, void* scratch, int64_t maxstates, int shuffle, uint64_t seed,
                     uint64_t step, const TruncWs& ws, uint64_t* out_keys, int* out_blk, int64_t out_cap, float* out_w,
-                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, cudaStream_t st);
+                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, int at_once, cudaStream_t st);
 
 }  // namespace paces
