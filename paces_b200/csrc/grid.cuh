@@ -23,8 +23,7 @@ __device__ __forceinline__ bool grid_barrier_warp(unsigned* bar, unsigned nblock
             ok = 0;
         } else {
             const unsigned target = (gen + 1) * nblocks;
-            __threadfence();
-            atomicAdd(bar, 1u);
+            asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
             const uint64_t t0 = global_ns();
             unsigned seen;
             for (;;) {
@@ -36,7 +35,6 @@ __device__ __forceinline__ bool grid_barrier_warp(unsigned* bar, unsigned nblock
                     break;
                 }
             }
-            __threadfence();
         }
     }
     return __shfl_sync(0xffffffffu, ok, 0) != 0;

@@ -547,10 +547,8 @@ __device__ long long lookback_warp(unsigned long long* state, int t, long long c
         if (first_inc < 32) break;
         top -= 32 * kLbPerLane;
     }
-    if (lane == 0) {
-        __threadfence();
-        atomicExch(&state[t], kLbInc | (unsigned long long)(excl + count));
-    }
+    // the word carries all that a later tile takes from this one: nothing to order it with
+    if (lane == 0) atomicExch(&state[t], kLbInc | (unsigned long long)(excl + count));
     return excl;
 }
 
