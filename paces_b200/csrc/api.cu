@@ -290,8 +290,11 @@ LanczosWs lanczos_ws(const paces_ctx* c, void* krylov, int64_t cap, int order) {
 bool valid_basis(const paces_basis* b) { return b && b->keys && b->blk && b->cap >= 0; }
 
 __global__ void record_init_kernel(paces_step_record* rec, int diagnostics) {
+    static_assert(sizeof(paces_step_record) % sizeof(int) == 0, "the record is cleared by words");
+    for (int i = threadIdx.x; i < int(sizeof(paces_step_record) / sizeof(int)); i += blockDim.x)
+        reinterpret_cast<int*>(rec)[i] = 0;
+    __syncthreads();
     if (threadIdx.x != 0) return;
-    memset(rec, 0, sizeof(paces_step_record));
     rec->post_adapt_norm = -1.0;
     rec->post_adapt_energy_re = __longlong_as_double(0x7ff8000000000000ll);
     rec->post_adapt_energy_im = 0.0;
@@ -441,7 +444,7 @@ int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks, int at_on
     auto mark = [&](int i) {
         if (marks && c->profiling) cudaEventRecord(c->ev[i], st);
     };
-    record_init_kernel<<<1, 32, 0, st>>>(rec, prm->diagnostics);
+    record_init_kernel<<<1, 256, 0, st>>>(rec, prm->diagnostics);
     mark(0);
     // 1. truncation of the old state (ranked by the look-ahead weights, in the Taylor term
     //    buffer, which is free until the propagation)
