@@ -114,6 +114,36 @@ __device__ __forceinline__ int key_cmp(const Key<NW>& a, const Key<NW>& b) {
     return 0;
 }
 
+// ~0 when a < b, else 0: the borrow of a - b, over one word or two.
+__device__ __forceinline__ uint32_t below(uint64_t a, uint64_t b) {
+    uint32_t r;
+    asm("{\n\t.reg .u64 t;\n\tsub.cc.u64 t, %1, %2;\n\tsubc.u32 %0, 0, 0;\n\t}" : "=r"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t below(uint64_t ah, uint64_t al, uint64_t bh, uint64_t bl) {
+    uint32_t r;
+    asm("{\n\t.reg .u64 t;\n\tsub.cc.u64 t, %2, %4;\n\tsubc.cc.u64 t, %1, %3;\n\tsubc.u32 %0, 0, 0;\n\t}"
+        : "=r"(r)
+        : "l"(ah), "l"(al), "l"(bh), "l"(bl));
+    return r;
+}
+
+// a < b, without branches on where the keys first differ (a warp's lanes differ in different
+// words).  In the remap's searches against a word-by-word compare that returns early: 256 -> 211 us
+// at 15.2M two-word rows, 86 -> 79 at 4.0M, 63 -> 55 at 1.4M one-word rows; equal at four words.
+template <int NW>
+__device__ __forceinline__ bool key_below(const Key<NW>& a, const Key<NW>& b) {
+    uint32_t lt = 0;
+    if constexpr (NW % 2 == 1) lt = below(a.w[NW - 1], b.w[NW - 1]);
+#pragma unroll
+    for (int q = NW - 2 - NW % 2; q >= 0; q -= 2) {
+        const uint32_t c = below(a.w[q], a.w[q + 1], b.w[q], b.w[q + 1]);
+        if (q == NW - 2) lt = c;
+        else lt = c | ((a.w[q] == b.w[q] && a.w[q + 1] == b.w[q + 1]) ? lt : 0u);
+    }
+    return lt != 0;
+}
+
 template <int NW>
 __device__ __forceinline__ bool key_eq(const Key<NW>& a, const Key<NW>& b) {
     bool eq = true;

@@ -27,7 +27,7 @@ __device__ int merge_path(const uint64_t* __restrict__ A, int na, const uint64_t
         const int mid = (begin + end) >> 1;
         const Key<NW> a = load_key<NW>(A, mid);
         const Key<NW> b = load_key<NW>(B, diag - 1 - mid);
-        if (!(key_cmp(b, a) < 0)) begin = mid + 1; else end = mid;
+        if (!key_below(b, a)) begin = mid + 1; else end = mid;
     }
     return begin;
 }
@@ -132,18 +132,18 @@ __global__ void __launch_bounds__(kRThreads) remap_tile_kernel(ModelDev m, const
             if (u == 0) {
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
-                    if (key_cmp(s_old[h + mid], k) <= 0) lo = mid + 1; else hi = mid;
+                    if (!key_below(k, s_old[h + mid])) lo = mid + 1; else hi = mid;
                 }
             } else {
                 int steps = 0;
-                while (lo < nold && steps < 8 && key_cmp(s_old[h + lo], k) <= 0) {
+                while (lo < nold && steps < 8 && !key_below(k, s_old[h + lo])) {
                     ++lo;
                     ++steps;
                 }
                 if (steps == 8)
                     while (lo < hi) {
                         const int mid = (lo + hi) >> 1;
-                        if (key_cmp(s_old[h + mid], k) <= 0) lo = mid + 1; else hi = mid;
+                        if (!key_below(k, s_old[h + mid])) lo = mid + 1; else hi = mid;
                     }
             }
             const int aa = a0 + lo;  // old elements before k in merged order
