@@ -29,47 +29,61 @@ __device__ __forceinline__ int run_source(const ModelDev& m, const MergeWs& ws, 
     return p;
 }
 
-// Element `src` of X as it appears in run j of block p: key and order flag
+// The exciton site's field of a block: where the phonon runs change a key.  Read from the model
+// once per block, not per element (the lookups by site are dependent constant loads): the tile
+// kernels are bound by the instructions they issue.  With the comparisons by borrow and the
+// transforms without branches, expand 646 -> 626 and assemble 1067 -> 1049 us at 4.2M kept states.
+struct SiteField {
+    int w, sh;        // its word and bit
+    uint32_t mask, top;  // the field's mask and largest occupation
+    uint64_t one, low;   // one phonon, and the bits below the field
+};
+__device__ __forceinline__ SiteField site_field(const ModelDev& m, int p) {
+    SiteField s;
+    s.w = m.word[p];
+    s.sh = m.shift[p];
+    s.mask = (1u << m.bits[p]) - 1u;
+    s.top = uint32_t(m.maxd[p]) - 1u;
+    s.one = uint64_t(1) << s.sh;
+    s.low = s.one - 1;
+    return s;
+}
+
+// Element `src` of X as it appears in run j of the site's block: key and order flag
 // (0 = floor hole, 1 = real, 2 = ceiling hole).
 template <int NW>
-__device__ __forceinline__ void run_transform(const ModelDev& m, const MergeWs& ws, int p, int j, int64_t src,
-                                              Key<NW>& k, int& flag) {
+__device__ __forceinline__ void run_transform(const SiteField& s, const MergeWs& ws, int j, int64_t src, Key<NW>& k,
+                                              int& flag) {
     flag = 1;
     if (ws.keep && j != RUN_SELF && src < ws.keep_cap && !__ldg(ws.keep + j * ws.keep_cap + src)) flag = 2;
     const int kind = ws.run_kind[j];
-    if (kind == RK_UP || kind == RK_DOWN) {
-        const int w = m.word[p];
-        const int sh = m.shift[p];
-        const uint32_t n = get_field(m, k, p);
-        const uint64_t low = sh == 0 ? 0ull : ((uint64_t(1) << sh) - 1);
-        if (kind == RK_UP) {
-            if (n + 1 >= m.maxd[p]) {
-                flag = 2;
+    if (kind != RK_UP && kind != RK_DOWN) return;
+    // a mask per word instead of a select on the word index (see get_field)
+    uint64_t word = 0;
 #pragma unroll
-                for (int q = 0; q < NW; ++q)
-                    k.w[q] = (k.w[q] | (low & (0ull - uint64_t(q == w)))) | (0ull - uint64_t(q > w));
-            } else {
-                add_field(m, k, p, +1);
-            }
-        } else {
-            if (n == 0) {
-                flag = 0;
+    for (int q = 0; q < NW; ++q) word |= k.w[q] & (0ull - uint64_t(q == s.w));
+    const uint32_t n = uint32_t(word >> s.sh) & s.mask;
+    const bool up = kind == RK_UP;
+    const bool hole = up ? n >= s.top : n == 0;
+    const uint64_t add = hole ? 0ull : (up ? s.one : 0ull - s.one);
+    if (hole) flag = up ? 2 : 0;
+    // a hole: every bit below the field set (up) or cleared (down)
+    const uint64_t low = hole ? s.low : 0ull, rest = hole ? ~0ull : 0ull;
 #pragma unroll
-                for (int q = 0; q < NW; ++q)
-                    k.w[q] = (k.w[q] & ~(low & (0ull - uint64_t(q == w)))) & ~(0ull - uint64_t(q > w));
-            } else {
-                add_field(m, k, p, -1);
-            }
-        }
+    for (int q = 0; q < NW; ++q) {
+        const uint64_t at = 0ull - uint64_t(q == s.w);
+        const uint64_t fill = (low & at) | (rest & (0ull - uint64_t(q > s.w)));
+        const uint64_t v = k.w[q] + (add & at);
+        k.w[q] = up ? v | fill : v & ~fill;
     }
 }
 
 template <int NW>
-__device__ __forceinline__ void run_elem(const ModelDev& m, const uint64_t* __restrict__ X,
-                                         const uint64_t* __restrict__ Y, const MergeWs& ws, int p, int j,
-                                         int64_t src, Key<NW>& k, int& flag) {
+__device__ __forceinline__ void run_elem(const SiteField& s, const uint64_t* __restrict__ X,
+                                         const uint64_t* __restrict__ Y, const MergeWs& ws, int j, int64_t src, Key<NW>& k,
+                                         int& flag) {
     k = load_key<NW>(j == RUN_SELF ? X : Y, src);
-    run_transform<NW>(m, ws, p, j, src, k, flag);
+    run_transform<NW>(s, ws, j, src, k, flag);
 }
 
 template <int NW>
@@ -111,14 +125,21 @@ struct SKeys {
     }
 };
 
-// (key, flag) pairs held in registers: a strictly below b.  Branch-free fold from the least
-// significant word, so a warp's lanes never diverge on where their keys first differ.
+// (key, flag) pairs held in registers: a strictly below b, without branches.
 template <int NW>
 __device__ __forceinline__ bool reg_less(const Key<NW>& a, int fa, const Key<NW>& b, int fb) {
-    bool lt = fa < fb;
-#pragma unroll
-    for (int q = NW - 1; q >= 0; --q) lt = (a.w[q] < b.w[q]) | ((a.w[q] == b.w[q]) & lt);
-    return lt;
+    if constexpr (NW == 1) {
+        return below(a.w[0], uint64_t(unsigned(fa)), b.w[0], uint64_t(unsigned(fb))) != 0;
+    } else if constexpr (NW == 2) {
+        uint32_t r;  // the borrow of (a, fa) - (b, fb)
+        asm("{\n\t.reg .u32 f;\n\t.reg .u64 t;\n\tsub.cc.u32 f, %5, %6;\n\tsubc.cc.u64 t, %2, %4;\n\t"
+            "subc.cc.u64 t, %1, %3;\n\tsubc.u32 %0, 0, 0;\n\t}"
+            : "=r"(r)
+            : "l"(a.w[0]), "l"(a.w[1]), "l"(b.w[0]), "l"(b.w[1]), "r"(fa), "r"(fb));
+        return r != 0;
+    } else {
+        return key_below(a, b) | (key_eq(a, b) & (fa < fb));
+    }
 }
 
 template <int NW>
@@ -443,7 +464,8 @@ __global__ void __launch_bounds__(256) merge_split_kernel(ModelDev m, const uint
         const int i = (s - s_off[r]) * stride;
         Key<NW> k;
         int f;
-        run_elem<NW>(m, X, Y, ws, p, j, s_lo[r] + i, k, f);
+        const SiteField site = site_field(m, p);
+        run_elem<NW>(site, X, Y, ws, j, s_lo[r] + i, k, f);
         // the bounds in the other runs: all searches advance one step per round, so their
         // dependent loads are in flight together
         int lo_[kRuns], a_[kRuns], b_[kRuns];
@@ -462,9 +484,11 @@ __global__ void __launch_bounds__(256) merge_split_kernel(ModelDev m, const uint
                 const int mid = (a_[jj] + b_[jj]) >> 1;
                 Key<NW> k2;
                 int f2;
-                run_elem<NW>(m, X, Y, ws, p, jj, lo_[jj] + mid, k2, f2);
-                const int c = cmp_kf(k2, f2, k, f);
-                if ((jj < j) ? (c <= 0) : (c < 0)) a_[jj] = mid + 1; else b_[jj] = mid;
+                run_elem<NW>(site, X, Y, ws, jj, lo_[jj] + mid, k2, f2);
+                // before this splitter: smaller, or equal in an earlier run
+                const bool same = key_eq(k2, k);
+                const bool before = key_below(k2, k) | (same & (f2 < f || (f2 == f && jj < j)));
+                if (before) a_[jj] = mid + 1; else b_[jj] = mid;
             }
             if (!any) break;
         }
@@ -625,7 +649,7 @@ __device__ __forceinline__ void tile_setup(const ModelDev& m, const uint64_t* __
 #pragma unroll
     for (int q = 0; q < NW; ++q) mine.w[q] = 0;
     const bool has = lane < kRuns && ok && start > 0;
-    if (has) run_elem<NW>(m, X, Y, ws, p, lane, int64_t(lo) + start - 1, mine, minef);
+    if (has) run_elem<NW>(site_field(m, p), X, Y, ws, lane, int64_t(lo) + start - 1, mine, minef);
     const unsigned any = __ballot_sync(0xffffffffu, has);
     Key<NW> pk = mine;
     int pf = minef;
@@ -776,6 +800,7 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
 #pragma unroll
         for (int q = 0; q < NW; ++q) s_pred.w[q] = s_d.pred[q];
 
+        const SiteField site = site_field(m, p);
         // transforms applied in place
         if constexpr (NW % 2 == 0) {
             const uint32_t mb = tc::smem_addr(&s_mbar);
@@ -793,7 +818,7 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
                 int f = 1;
                 if (kind == RK_UP || kind == RK_DOWN || (ws.keep && j != RUN_SELF)) {
                     Key<NW> k = s_key.get(e);
-                    run_transform<NW>(m, ws, p, j, int64_t(s_lo[j]) + s_start[j] + (e - s_off[j]), k, f);
+                    run_transform<NW>(site, ws, j, int64_t(s_lo[j]) + s_start[j] + (e - s_off[j]), k, f);
                     s_key.set(e, k);
                 }
                 s_flag[e] = uint8_t(f);
@@ -805,7 +830,7 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
                 for (int q = 1; q < kRuns; ++q) j += (e >= s_off[q]);
                 Key<NW> k;
                 int f;
-                run_elem<NW>(m, X, Y, ws, p, j, int64_t(s_lo[j]) + s_start[j] + (e - s_off[j]), k, f);
+                run_elem<NW>(site, X, Y, ws, j, int64_t(s_lo[j]) + s_start[j] + (e - s_off[j]), k, f);
                 s_key.set(e, k);
                 s_flag[e] = uint8_t(f);
             }
