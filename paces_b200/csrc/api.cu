@@ -173,7 +173,8 @@ ModelDev with_h(const paces_ctx* c, const paces_hmat* h) {
     return m;
 }
 
-MergeWs merge_ws(const paces_ctx* c, const Layout& l, void* ws) {
+// at_once: merges that share the device, each cut for its share of the SMs
+MergeWs merge_ws(const paces_ctx* c, const Layout& l, void* ws, int at_once = 1) {
     MergeWs w;
     w.run_lo = at<int>(ws, l.m_run_lo);
     w.run_len = at<int>(ws, l.m_run_len);
@@ -183,6 +184,8 @@ MergeWs merge_ws(const paces_ctx* c, const Layout& l, void* ws) {
     w.ord_co = at<int>(ws, l.m_ord_co);
     w.tile_state = at<unsigned long long>(ws, l.m_tile_state);
     w.split_cap = int(l.split_cap);
+    w.want_splits = merge_want_splits(c->num_sms) / at_once;
+    w.wide_splits = kWideSplitters / at_once;
     w.tile_cap = int(l.tile_cap);
     w.keep = nullptr;
     w.keep_cap = 0;
@@ -519,7 +522,7 @@ int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks, int at_on
         p.enl_blk = bufs[ci].blk;
     }
     for (int e = 0; e < prm->enlarge_steps && !multi; ++e) {
-        MergeWs mws = merge_ws(c, l, ws);
+        MergeWs mws = merge_ws(c, l, ws, at_once);
         if (propose && e == 0) {
             mws.keep = at<uint8_t>(ws, l.keep);
             mws.keep_cap = l.cap;
@@ -564,7 +567,7 @@ int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks, int at_on
         mo.self_flag = at<uint8_t>(ws, l.v_TA);
         if (mo.cap > self_flag_cap(c, l)) mo.cap = self_flag_cap(c, l);
         PACES_CHECK_LAUNCH(c, launch_merge(c->nw, MERGE_ASSEMBLE, c->assemble_stride, c->m, cur->keys, cur->blk,
-                                           split ? nbasis.keys : nullptr, split ? nbasis.blk : nullptr, merge_ws(c, l, ws),
+                                           split ? nbasis.keys : nullptr, split ? nbasis.blk : nullptr, merge_ws(c, l, ws, at_once),
                                            mo, &rec->ceiling_hits, split ? 1 : 0, status, c->num_sms, st),
                            "step/assemble");
         if (split)

@@ -49,14 +49,16 @@ __device__ __forceinline__ SiteField site_field(const ModelDev& m, int p) {
     return s;
 }
 
-// Element `src` of X as it appears in run j of the site's block: key and order flag
+// Whether element `src` takes part in run j (proposals may leave some out).
+__device__ __forceinline__ bool run_keeps(const MergeWs& ws, int j, int64_t src) {
+    return !(ws.keep && j != RUN_SELF && src < ws.keep_cap) || __ldg(ws.keep + j * ws.keep_cap + src) != 0;
+}
+
+// An element of X as it appears in a run of the site's block: key and order flag
 // (0 = floor hole, 1 = real, 2 = ceiling hole).
 template <int NW>
-__device__ __forceinline__ void run_transform(const SiteField& s, const MergeWs& ws, int j, int64_t src, Key<NW>& k,
-                                              int& flag) {
-    flag = 1;
-    if (ws.keep && j != RUN_SELF && src < ws.keep_cap && !__ldg(ws.keep + j * ws.keep_cap + src)) flag = 2;
-    const int kind = ws.run_kind[j];
+__device__ __forceinline__ void run_transform(const SiteField& s, int kind, bool keeps, Key<NW>& k, int& flag) {
+    flag = keeps ? 1 : 2;
     if (kind != RK_UP && kind != RK_DOWN) return;
     // a mask per word instead of a select on the word index (see get_field)
     uint64_t word = 0;
@@ -83,7 +85,7 @@ __device__ __forceinline__ void run_elem(const SiteField& s, const uint64_t* __r
                                          const uint64_t* __restrict__ Y, const MergeWs& ws, int j, int64_t src, Key<NW>& k,
                                          int& flag) {
     k = load_key<NW>(j == RUN_SELF ? X : Y, src);
-    run_transform<NW>(s, ws, j, src, k, flag);
+    run_transform<NW>(s, ws.run_kind[j], run_keeps(ws, j, src), k, flag);
 }
 
 template <int NW>
@@ -371,23 +373,92 @@ __device__ __forceinline__ int merge_range_first(const SKeys<NW>& keys, const ui
     return c | (cn << 16);
 }
 
+// The splitters' bounds, one thread per splitter: all its searches advance one step per round,
+// kProbe runs' loads in flight together before the first compare.  (Each run's load behind the
+// last run's compare: 2200 cycles a round instead of 1700, 40 -> 27 us a launch at 524K four-word
+// states.)
+template <int NW>
+__device__ __forceinline__ void split_by_thread(const ModelDev& m, const uint64_t* __restrict__ X,
+                                                const uint64_t* __restrict__ Y, const MergeWs& ws, const int* s_off,
+                                                const int* s_lo, const int* s_len, int nr, int total, int stride) {
+    constexpr int kProbe = NW <= 4 ? kRuns : 20 / NW;
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < total; s += gridDim.x * blockDim.x) {
+        const int r = find_segment(s_off, nr, s);
+        const int p = r / kRuns, j = r % kRuns;
+        const int i = (s - s_off[r]) * stride;
+        Key<NW> k;
+        int f;
+        const SiteField site = site_field(m, p);
+        run_elem<NW>(site, X, Y, ws, j, s_lo[r] + i, k, f);
+        int lo_[kRuns], a_[kRuns], b_[kRuns];
+#pragma unroll
+        for (int jj = 0; jj < kRuns; ++jj) {
+            lo_[jj] = s_lo[p * kRuns + jj];
+            a_[jj] = 0;
+            b_[jj] = jj == j ? 0 : s_len[p * kRuns + jj];
+        }
+        for (;;) {
+            bool any = false;
+#pragma unroll
+            for (int j0 = 0; j0 < kRuns; j0 += kProbe) {
+                Key<NW> k2[kProbe];
+                bool keeps[kProbe];
+#pragma unroll
+                for (int u = 0; u < kProbe; ++u) {
+                    const int jj = j0 + u;
+                    if (jj >= kRuns) continue;
+                    keeps[u] = true;
+                    if (a_[jj] < b_[jj]) {
+                        const int64_t src = lo_[jj] + ((a_[jj] + b_[jj]) >> 1);
+                        k2[u] = load_key<NW>(jj == RUN_SELF ? X : Y, src);
+                        keeps[u] = run_keeps(ws, jj, src);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kProbe; ++u) {
+                    const int jj = j0 + u;
+                    if (jj >= kRuns || a_[jj] >= b_[jj]) continue;
+                    any = true;
+                    int f2;
+                    run_transform<NW>(site, ws.run_kind[jj], keeps[u], k2[u], f2);
+                    // before this splitter: smaller, or equal in an earlier run
+                    const bool same = key_eq(k2[u], k);
+                    const bool before = key_below(k2[u], k) | (same & (f2 < f || (f2 == f && jj < j)));
+                    const int mid = (a_[jj] + b_[jj]) >> 1;
+                    if (before) a_[jj] = mid + 1; else b_[jj] = mid;
+                }
+            }
+            if (!any) break;
+        }
+        int dst = s_off[p * kRuns];
+#pragma unroll
+        for (int jj = 0; jj < kRuns; ++jj) {
+            if (jj == j) a_[jj] = i;
+            dst += (a_[jj] + stride - 1) / stride;
+        }
+        if (dst >= s_off[(p + 1) * kRuns]) continue;  // inconsistent ranks: cannot happen for sorted runs
+#pragma unroll
+        for (int jj = 0; jj < kRuns; ++jj) ws.ord_co[int64_t(dst) * kRuns + jj] = a_[jj];
+    }
+}
+
 // Splitters every `stride` elements of each run, with their co-ranks in the block's other
 // runs.  The plan comes first and every block derives it from the block offsets: the runs'
 // extents, the splitter prefix over (block, run) and the tile prefix over blocks (a tile is
 // kMergeGroup splitter intervals of one block).  Block 0 publishes it, sets the counters and
 // every block clears its share of the look-back words for the tile kernel.
 template <int NW>
-__global__ void __launch_bounds__(256) merge_split_kernel(ModelDev m, const uint64_t* __restrict__ X,
+__global__ void __launch_bounds__(256, NW <= 2 ? 4 : 2) merge_split_kernel(ModelDev m, const uint64_t* __restrict__ X,
                                                           const uint64_t* __restrict__ Y,
                                                           const int* __restrict__ x_blk,
-                                                          const int* __restrict__ y_blk, MergeWs ws, int stride,
-                                                          int* status) {
+                                                          const int* __restrict__ y_blk, MergeWs ws,
+                                                          int max_stride, int* status) {
     __shared__ int s_lo[kMaxSites * kRuns];
     __shared__ int s_len[kMaxSites * kRuns];
     __shared__ int s_off[kMaxSites * kRuns + 1];
     __shared__ int s_pos[kMaxSites + 1];  // splitters per block, then their prefix
     __shared__ int s_toff[kMaxSites + 1];
-    __shared__ int s_total, s_tiles;
+    __shared__ int s_total, s_tiles, s_stride;
     const int L = m.L;
     const int nr = L * kRuns;
     for (int idx = threadIdx.x; idx < nr; idx += blockDim.x) {
@@ -403,6 +474,16 @@ __global__ void __launch_bounds__(256) merge_split_kernel(ModelDev m, const uint
         s_len[idx] = len;
     }
     __syncthreads();
+    if (threadIdx.x < 32) {
+        int64_t elems = 0;
+        for (int idx = threadIdx.x; idx < nr; idx += 32) elems += s_len[idx];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) elems += __shfl_xor_sync(0xffffffffu, elems, o);
+        if (threadIdx.x == 0)
+            s_stride = int(min(int64_t(max_stride), max(int64_t(kSmallMergeStride), elems / max(ws.want_splits, 1) + 1)));
+    }
+    __syncthreads();
+    const int stride = s_stride;
     for (int p = threadIdx.x; p < L; p += blockDim.x) {
         int c = 0;
 #pragma unroll
@@ -410,28 +491,42 @@ __global__ void __launch_bounds__(256) merge_split_kernel(ModelDev m, const uint
         s_pos[p] = c;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         int acc = 0, tacc = 0;
-        for (int p = 0; p < L; ++p) {
-            const int c = s_pos[p];
-            s_pos[p] = acc;
-            s_toff[p] = tacc;
-            acc += c;
-            tacc += (c + kMergeGroup - 1) / kMergeGroup;
+        for (int p0 = 0; p0 < L; p0 += 32) {
+            const int p = p0 + int(threadIdx.x);
+            const int c = p < L ? s_pos[p] : 0, tc = (c + kMergeGroup - 1) / kMergeGroup;
+            int incl = c, tincl = tc;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o), tv = __shfl_up_sync(0xffffffffu, tincl, o);
+                if (int(threadIdx.x) >= o) {
+                    incl += v;
+                    tincl += tv;
+                }
+            }
+            if (p < L) {
+                s_pos[p] = acc + incl - c;
+                s_toff[p] = tacc + tincl - tc;
+            }
+            acc += __shfl_sync(0xffffffffu, incl, 31);
+            tacc += __shfl_sync(0xffffffffu, tincl, 31);
         }
-        s_pos[L] = acc;
-        s_toff[L] = tacc;
-        const bool ok = acc <= ws.split_cap && tacc <= ws.tile_cap;
-        s_total = ok ? acc : 0;
-        s_tiles = ok ? tacc : 0;
-        if (blockIdx.x == 0) {
-            if (!ok) raise_status(status, PACES_ERR_CAPACITY);
-            ws.counters[0] = s_total;
-            ws.counters[1] = s_tiles;
-            ws.counters[2] = 0;
-            ws.counters[3] = 0;
-            ws.counters[4] = 0;
-            ws.counters[5] = 0;
+        if (threadIdx.x == 0) {
+            s_pos[L] = acc;
+            s_toff[L] = tacc;
+            const bool ok = acc <= ws.split_cap && tacc <= ws.tile_cap;
+            s_total = ok ? acc : 0;
+            s_tiles = ok ? tacc : 0;
+            if (blockIdx.x == 0) {
+                if (!ok) raise_status(status, PACES_ERR_CAPACITY);
+                ws.counters[0] = s_total;
+                ws.counters[1] = s_tiles;
+                ws.counters[2] = 0;
+                ws.counters[3] = 0;
+                ws.counters[4] = 0;
+                ws.counters[5] = 0;
+            }
         }
     }
     __syncthreads();
@@ -458,7 +553,15 @@ __global__ void __launch_bounds__(256) merge_split_kernel(ModelDev m, const uint
         ws.tile_state[t] = 0ull;
 
     const int total = s_total;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < total; s += gridDim.x * blockDim.x) {
+    if (total > ws.wide_splits) {
+        split_by_thread<NW>(m, X, Y, ws, s_off, s_lo, s_len, nr, total, stride);
+        return;
+    }
+    const int jj = threadIdx.x & 7;
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    const int kind = jj < kRuns ? ws.run_kind[jj] : RK_EMPTY;
+    const uint64_t* run = jj == RUN_SELF ? X : Y;
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; s < total; s += (gridDim.x * blockDim.x) >> 3) {
         const int r = find_segment(s_off, nr, s);
         const int p = r / kRuns, j = r % kRuns;
         const int i = (s - s_off[r]) * stride;
@@ -466,43 +569,40 @@ __global__ void __launch_bounds__(256) merge_split_kernel(ModelDev m, const uint
         int f;
         const SiteField site = site_field(m, p);
         run_elem<NW>(site, X, Y, ws, j, s_lo[r] + i, k, f);
-        // the bounds in the other runs: all searches advance one step per round, so their
-        // dependent loads are in flight together
-        int lo_[kRuns], a_[kRuns], b_[kRuns];
-#pragma unroll
-        for (int jj = 0; jj < kRuns; ++jj) {
-            lo_[jj] = s_lo[p * kRuns + jj];
-            a_[jj] = 0;
-            b_[jj] = jj == j ? 0 : s_len[p * kRuns + jj];
+        int a = 0, b = 0, lo = 0;
+        if (jj < kRuns && jj != j) {
+            lo = s_lo[p * kRuns + jj];
+            b = s_len[p * kRuns + jj];
         }
-        for (;;) {
-            bool any = false;
+        while (a < b) {
+            const int n = b - a, at[3] = {a + (n >> 2), a + (n >> 1), a + (n >> 1) + (n >> 2)};
+            Key<NW> kq[3];
+            bool keeps[3], before[3];
 #pragma unroll
-            for (int jj = 0; jj < kRuns; ++jj) {
-                if (a_[jj] >= b_[jj]) continue;
-                any = true;
-                const int mid = (a_[jj] + b_[jj]) >> 1;
-                Key<NW> k2;
-                int f2;
-                run_elem<NW>(site, X, Y, ws, jj, lo_[jj] + mid, k2, f2);
-                // before this splitter: smaller, or equal in an earlier run
-                const bool same = key_eq(k2, k);
-                const bool before = key_below(k2, k) | (same & (f2 < f || (f2 == f && jj < j)));
-                if (before) a_[jj] = mid + 1; else b_[jj] = mid;
+            for (int u = 0; u < 3; ++u) {
+                kq[u] = load_key<NW>(run, lo + at[u]);
+                keeps[u] = run_keeps(ws, jj, lo + at[u]);
             }
-            if (!any) break;
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                int fq;
+                run_transform<NW>(site, kind, keeps[u], kq[u], fq);
+                // before this splitter: smaller, or equal in an earlier run
+                before[u] = key_below(kq[u], k) | (key_eq(kq[u], k) & ((fq < f) | ((fq == f) & (jj < j))));
+            }
+            const int na = before[2] ? at[2] + 1 : (before[1] ? at[1] + 1 : (before[0] ? at[0] + 1 : a));
+            b = before[2] ? b : (before[1] ? at[2] : (before[0] ? at[1] : at[0]));
+            a = na;
         }
         // its place among the block's splitters in merged order: run jj has a splitter every
         // `stride` elements, so ceil(co / stride) of them lie before co of its elements
-        int dst = s_off[p * kRuns];
+        if (jj == j) a = i;
+        int dst = (a + stride - 1) / stride;
 #pragma unroll
-        for (int jj = 0; jj < kRuns; ++jj) {
-            if (jj == j) a_[jj] = i;
-            dst += (a_[jj] + stride - 1) / stride;
-        }
+        for (int o = 4; o > 0; o >>= 1) dst += __shfl_xor_sync(group, dst, o);
+        dst += s_off[p * kRuns];
         if (dst >= s_off[(p + 1) * kRuns]) continue;  // inconsistent ranks: cannot happen for sorted runs
-#pragma unroll
-        for (int jj = 0; jj < kRuns; ++jj) ws.ord_co[int64_t(dst) * kRuns + jj] = a_[jj];
+        if (jj < kRuns) ws.ord_co[int64_t(dst) * kRuns + jj] = a;
     }
 }
 
@@ -818,7 +918,7 @@ merge_tile_kernel(ModelDev m, const uint64_t* __restrict__ X, const uint64_t* __
                 int f = 1;
                 if (kind == RK_UP || kind == RK_DOWN || (ws.keep && j != RUN_SELF)) {
                     Key<NW> k = s_key.get(e);
-                    run_transform<NW>(site, ws, j, int64_t(s_lo[j]) + s_start[j] + (e - s_off[j]), k, f);
+                    run_transform<NW>(site, kind, run_keeps(ws, j, int64_t(s_lo[j]) + s_start[j] + (e - s_off[j])), k, f);
                     s_key.set(e, k);
                 }
                 s_flag[e] = uint8_t(f);
@@ -1096,7 +1196,7 @@ int launch_merge_t(int mode, int stride, const ModelDev& m, const uint64_t* X, c
     const int tmax = merge_tmax(stride);
     MergeOut o = out;
     if (mode == MERGE_ASSEMBLE && !split_input && out.nbr) o.self_rows_filled = 1;  // nbr_fill_kernel below
-    const int g = grid_for(ws.split_cap, 256, num_sms * 8);
+    const int g = grid_for(int64_t(ws.split_cap) * 8, 256, num_sms * 8);  // eight lanes per splitter
     merge_split_kernel<NW><<<g, 256, 0, st>>>(m, X, Y, x_blk, y_blk, ws, stride, status);
     if (mode == MERGE_ASSEMBLE)
         launch_tile<NW, MERGE_ASSEMBLE>(tmax, m, X, Y, ws, o, ceiling_out, ceiling_add, status, num_sms, st);

@@ -45,6 +45,8 @@ struct MergeWs {
     unsigned long long* tile_state;  // [tile_cap] look-back words
     int split_cap;
     int tile_cap;
+    int want_splits;  // small inputs are cut into about this many splitter intervals (see kSmallMergeStride)
+    int wide_splits;  // up to this many splitters, eight lanes search for each (see kWideSplitters)
     // optional candidate filter (expansion only): keep[j * keep_cap + src] == 0 drops the
     // image of source element src under run j (j = 1..4); dropped images sort like
     // ceiling holes (after real elements with the same key) and are never emitted
@@ -139,10 +141,29 @@ constexpr int kMergeGroup = 12;
 // (kMergeGroup + kRuns) * stride elements in total.
 __host__ __device__ constexpr int merge_tmax(int stride) { return (kMergeGroup + kRuns) * stride; }
 
-// Splitter capacity for inputs of up to in_cap states at any stride >= kMinMergeStride.
+// Inputs too small to fill the SMs with tiles of the tuned stride are cut finer, down to this
+// stride, towards two tiles per SM: expand 52 -> 48 us and assemble 64 -> 57 us at 65K kept states,
+// 34 -> 33 and 44 -> 39 us at 4K.
+constexpr int kSmallMergeStride = 32;
+constexpr int kWantSplitsMax = 4096;
+inline int merge_want_splits(int num_sms) {
+    const int w = 2 * kMergeGroup * num_sms;
+    return w > kWantSplitsMax ? kWantSplitsMax : w;
+}
+
+// Up to this many splitters, eight lanes work on each: lane j searches run j, three probes a round
+// with their loads in flight together, half the rounds of a bisection.  Latency is all that counts
+// there: 19.6 -> 8.9 us a launch at 4K states (137 splitters), 115 -> 110 us for an assembly with
+// 15.2K.  With more of them the probes' traffic counts: at 19K splitters the assembly took 225 us
+// so and 218 us with a thread per splitter, at 33K 207 and 195 us.  Merges that run at once share
+// the line.
+constexpr int kWideSplitters = 16384;
+
+// Splitter capacity for inputs of up to in_cap states at any stride >= kMinMergeStride, and for
+// kWantSplitsMax intervals of smaller ones.
 inline int64_t merge_split_cap(int64_t in_cap, int nw, int L) {
     (void)nw;
-    return kRuns * (in_cap / kMinMergeStride + 1) + int64_t(kRuns) * L + 8;
+    return kRuns * (in_cap / kMinMergeStride + 1) + int64_t(kRuns) * L + 8 + kWantSplitsMax;
 }
 inline int64_t merge_tile_cap(int64_t split_cap, int L) { return split_cap / kMergeGroup + L + 8; }
 
