@@ -292,7 +292,12 @@ LanczosWs lanczos_ws(const paces_ctx* c, void* krylov, int64_t cap, int order) {
 
 bool valid_basis(const paces_basis* b) { return b && b->keys && b->blk && b->cap >= 0; }
 
-__global__ void record_init_kernel(paces_step_record* rec, int diagnostics) {
+// The record's start values, and the counters that the truncation and the propagation start from
+// (two clearing copies of their own took 3 us of a small step).
+__global__ void __launch_bounds__(1024) step_init_kernel(paces_step_record* rec, int diagnostics, unsigned* hist, unsigned* barrier) {
+    static_assert(kTruncHistBytes % sizeof(unsigned) == 0 && kTaylorBarrierBytes % sizeof(unsigned) == 0, "by words");
+    for (int i = threadIdx.x; i < int(kTruncHistBytes / sizeof(unsigned)); i += blockDim.x) hist[i] = 0;
+    for (int i = threadIdx.x; i < int(kTaylorBarrierBytes / sizeof(unsigned)); i += blockDim.x) barrier[i] = 0;
     static_assert(sizeof(paces_step_record) % sizeof(int) == 0, "the record is cleared by words");
     for (int i = threadIdx.x; i < int(sizeof(paces_step_record) / sizeof(int)); i += blockDim.x)
         reinterpret_cast<int*>(rec)[i] = 0;
@@ -302,13 +307,6 @@ __global__ void record_init_kernel(paces_step_record* rec, int diagnostics) {
     rec->post_adapt_energy_re = __longlong_as_double(0x7ff8000000000000ll);
     rec->post_adapt_energy_im = 0.0;
     (void)diagnostics;
-}
-
-// (n_select is written by the truncation: with several merge passes its buffer is reused)
-__global__ void record_counts_kernel(paces_step_record* rec, const int* enl_blk, const int* new_blk, int L) {
-    if (threadIdx.x != 0) return;
-    rec->n_enlarged = enl_blk[L];
-    rec->n_states = new_blk[L];
 }
 
 // Expansion (assemble = false) or assembly of X over every hopping channel of a lattice:
@@ -427,12 +425,12 @@ int plan_step(paces_ctx* c, const paces_basis* old_b, const void* old_psi, paces
 }
 
 // Kernels one step enqueues (merge: 2 per pass, +1 for the neighbour table; truncation: see
-// trunc_launches, +1 with look-ahead weights; remap 2; observables 2 or 3; Taylor 1;
-// renormalisation 3; record 2).
+// trunc_launches, +1 with look-ahead weights; remap 2; observables 2 or 3; Taylor 1, +1 for its
+// diagnostics; renormalisation 3; the record's start 1).
 unsigned long long step_launches(const paces_step_params& prm, bool with_taylor, int passes) {
-    return 2 + (prm.weighting ? 1 : 0) + trunc_launches(prm.shuffle != 0) +
+    return 1 + (prm.weighting ? 1 : 0) + trunc_launches(prm.shuffle != 0) +
            (prm.proposal && prm.enlarge_steps > 0 ? 1 : 0) + 2ull * passes * (prm.enlarge_steps + 1) + 1 +
-           2 + (prm.diagnostics ? 2 : 0) +
+           2 + (diag_in_taylor(&prm) ? 1 : (prm.diagnostics ? 2 : 0)) +
            (prm.evolve ? (with_taylor ? 1 : 0) + (prm.renormalize ? 3 : 0) : 0) + 3;
 }
 
@@ -447,7 +445,7 @@ int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks, int at_on
     auto mark = [&](int i) {
         if (marks && c->profiling) cudaEventRecord(c->ev[i], st);
     };
-    record_init_kernel<<<1, 256, 0, st>>>(rec, prm->diagnostics);
+    step_init_kernel<<<1, 1024, 0, st>>>(rec, prm->diagnostics, at<unsigned>(ws, l.t_hist), at<unsigned>(ws, l.v_bar));
     mark(0);
     // 1. truncation of the old state (ranked by the look-ahead weights, in the Taylor term
     //    buffer, which is free until the propagation)
@@ -465,7 +463,7 @@ int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks, int at_on
                                           prm->maxstates,
                                           prm->shuffle, prm->shuffle_seed, prm->step_index, trunc_ws(l, ws), p.A.keys,
                                           p.A.blk, p.A.cap, at<float>(ws, l.aw), &rec->n_tied, &rec->n_select, status, c->num_sms, at_once,
-                                          st),
+                                          st, true),
                        "step/truncate");
     // 1b. learned proposal: score the truncated basis' images
     const bool propose = prm->proposal && prm->enlarge_steps > 0;
@@ -612,11 +610,10 @@ int step_back(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks) {
     auto mark = [&](int i) {
         if (marks && c->profiling) cudaEventRecord(c->ev[i], st);
     };
-    if (diag_in_taylor(prm)) {
-        ObsTarget t{&rec->post_adapt_norm, &rec->post_adapt_energy_re, &rec->post_adapt_energy_im, nullptr, nullptr};
-        PACES_CHECK_LAUNCH(c, launch_diag_final(at<double>(p.ws, p.l.diag), p.new_b->blk, c->m.L, p.l.cap, t, st),
+    const double* diag_chunks = nullptr;
+    if (diag_in_taylor(prm))
+        PACES_CHECK_LAUNCH(c, launch_diag_chunks(at<double>(p.ws, p.l.diag), p.new_b->blk, c->m.L, p.l.cap, &diag_chunks, st),
                            "step/diagnostics");
-    }
     if (prm->evolve && prm->renormalize) {
         ObsTarget t{&rec->norm, nullptr, nullptr, nullptr, nullptr};
         PACES_CHECK_LAUNCH(c, launch_observables(c->nw, c64, with_h(c, p.h), p.new_b->keys, p.new_b->blk, p.h->nbr, p.h->cap,
@@ -628,14 +625,16 @@ int step_back(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks) {
     mark(6);
     // 7. observables of the new state
     {
-        ObsTarget t{&rec->norm, &rec->energy_re, &rec->energy_im, rec->n_exc, rec->n_pho};
+        // n_select is written by the truncation: with several merge passes its buffer is reused
+        ObsTarget t{&rec->norm, &rec->energy_re, &rec->energy_im, rec->n_exc, rec->n_pho,
+                    p.enl_blk, p.new_b->blk, &rec->n_enlarged, &rec->n_states,
+                    diag_chunks, &rec->post_adapt_norm, &rec->post_adapt_energy_re, &rec->post_adapt_energy_im};
         PACES_CHECK_LAUNCH(c, launch_observables(c->nw, c64, with_h(c, p.h), p.new_b->keys, p.new_b->blk, p.h->nbr, p.h->cap,
                                                  p.h->meta, p.new_psi,
                                                  PACES_OBS_NORM | PACES_OBS_ENERGY | PACES_OBS_SITES, opart, t,
                                                  c->num_sms, st),
                            "step/observables");
     }
-    record_counts_kernel<<<1, 32, 0, st>>>(rec, p.enl_blk, p.new_b->blk, c->m.L);
     mark(7);
     if (cudaGetLastError() != cudaSuccess) return cuda_fail(c, "step/record");
     return PACES_OK;
@@ -1235,7 +1234,7 @@ int paces_step(paces_ctx* c, const paces_basis* old_b, const void* old_psi, pace
             if (diag_in_taylor(prm)) tw.diag = at<double>(ws, p.l.diag);
             PACES_CHECK_LAUNCH(c, launch_taylor(c->precision == PACES_C64, with_h(c, h), new_b->blk, h->nbr, h->cap,
                                                 h->meta, p.target, new_psi, prm->dt, prm->m_star, prm->tol, tw, o,
-                                                &rec->status, c->num_sms, c->taylor_bps, c->taylor_variant, st),
+                                                &rec->status, c->num_sms, c->taylor_bps, c->taylor_variant, st, true),
                                "step/taylor");
         }
     }
@@ -1478,7 +1477,7 @@ int paces_batch_step(paces_batch* b, const paces_batch_item* items, int32_t n, p
             TaylorOut o{&p.rec->converged, &p.rec->final_m, &p.rec->c1_plus_c2, &p.rec->term_ratio};
             if (launch_taylor(c->precision == PACES_C64, with_h(c, p.h), p.new_b->blk, p.h->nbr, p.h->cap, p.h->meta,
                               p.target, p.new_psi, prm->dt, prm->m_star, prm->tol, tw, o, &p.rec->status, c->num_sms,
-                              c->taylor_bps, c->taylor_variant, st) != PACES_OK)
+                              c->taylor_bps, c->taylor_variant, st, true) != PACES_OK)
                 return bfail(PACES_ERR_CUDA, "item %d: Taylor: %s", i, cudaGetErrorString(cudaGetLastError()));
             launches += 1;
         }

@@ -138,7 +138,8 @@ int launch_lanczos(bool c64, const ModelDev& m, const int* blk, const int* nbr, 
 int launch_taylor(bool c64, const ModelDev& m, const int* blk, const int* nbr, int64_t nbr_cap,
                   const uint32_t* meta, const void* v_in, void* res, double dt, int m_star,
                   double tol, const TaylorWs& ws, const TaylorOut& out, int* status, int num_sms,
-                  int blocks_per_sm, int variant, cudaStream_t st);
+                  int blocks_per_sm, int variant, cudaStream_t st,
+                  bool cleared = false);  // the caller has zeroed ws.barrier
 
 // ---- scaling and squaring (expm.cu) ---------------------------------------------------------
 // out[0] = trace(H), out[1] = max row 1-norm of H - *shift I (0 when shift is null),
@@ -205,10 +206,21 @@ struct ObsTarget {
     double* energy_im;
     double* n_exc;       // [L] or null
     double* n_pho;       // [L] or null
+    // the end of a step, in one more block of the last reduction: the sizes of the enlarged and
+    // the new basis (new_blk null: not a step), and the diagnostics from a diag buffer's chunk
+    // sums (diag_chunks null: none)
+    const int* enl_blk = nullptr;
+    const int* new_blk = nullptr;
+    int* n_enlarged = nullptr;
+    int* n_states = nullptr;
+    const double* diag_chunks = nullptr;
+    double* diag_norm = nullptr;
+    double* diag_energy_re = nullptr;
+    double* diag_energy_im = nullptr;
 };
-// Norm and energy from a diag buffer filled by the first sweep of a Taylor launch (rows:
-// blk[L]; cap: the buffer's row capacity).  Two launches.
-int launch_diag_final(const double* diag, const int* blk, int L, int64_t cap, const ObsTarget& out, cudaStream_t st);
+// The chunk sums of a diag buffer filled by the first sweep of a Taylor launch (rows: blk[L];
+// cap: the buffer's row capacity); returns where they are in `chunks`.
+int launch_diag_chunks(const double* diag, const int* blk, int L, int64_t cap, const double** chunks, cudaStream_t st);
 constexpr int kObsGridPerSm = 4;
 inline int obs_max_grid(int num_sms) { return num_sms * kObsGridPerSm; }
 int launch_observables(int nw, bool c64, const ModelDev& m, const uint64_t* keys, const int* blk,

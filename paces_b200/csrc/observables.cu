@@ -293,13 +293,38 @@ obs_sites_kernel(ModelDev m, const uint64_t* __restrict__ keys, const int* __res
     }
 }
 
+// A step's sizes and, from the diag buffer's chunk sums in a fixed order -- warp q sums value q:
+// lane l the chunks l, l + 32, ... in order, then the butterfly -- the norm (square root of the
+// sum of |v|^2) and energy after the adaptation.
+__device__ __forceinline__ void step_end(int L, const ObsTarget& t) {
+    if (threadIdx.x == 0) {
+        *t.n_enlarged = t.enl_blk[L];
+        *t.n_states = t.new_blk[L];
+    }
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (!t.diag_chunks || q >= 3) return;
+    const int64_t nch = (diag_groups(t.new_blk[L]) + kDiagChunk - 1) / kDiagChunk;
+    double acc = 0.0;
+    for (int64_t c = lane; c < nch; c += 32) acc = __dadd_rn(acc, t.diag_chunks[c * 3 + q]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    if (lane != 0) return;
+    if (q == 0) *t.diag_norm = sqrt(acc);
+    else if (q == 1) *t.diag_energy_re = acc;
+    else *t.diag_energy_im = acc;
+}
+
 // One block per output value: strided partial sums then a fixed-shape tree (deterministic).
-// v = 0 norm, 1-2 energy (energy pass), 3.. n_exc and n_pho (site pass).
+// v = 0 norm, 1-2 energy (energy pass), 3.. n_exc and n_pho (site pass), then step_end's block.
 __global__ void __launch_bounds__(256) obs_final_kernel(int L, int nb_e, const double* __restrict__ part_e,
                                                         int nb_s, const double* __restrict__ part_s,
                                                         ObsTarget t) {
     __shared__ double s_w[8];
     const int v = blockIdx.x;
+    if (v == 3 + 2 * L) {
+        step_end(L, t);
+        return;
+    }
     const bool from_e = v < 3 && nb_e > 0;
     const int stride = from_e ? 3 : 1 + 2 * L;
     const int col = from_e ? v : (v == 0 ? 0 : v - 2);
@@ -357,26 +382,6 @@ __global__ void __launch_bounds__(256) diag_chunk_kernel(const double* __restric
         double acc = 0.0;
         for (int w = 0; w < 8; ++w) acc = __dadd_rn(acc, s_w[w][threadIdx.x]);
         chunks[c * 3 + threadIdx.x] = acc;
-    }
-}
-
-// The chunk sums in a fixed order -- warp q sums value q: lane l the chunks l, l + 32, ... in
-// order, then the butterfly -- into the norm (square root of the sum of |v|^2) and energy.
-__global__ void __launch_bounds__(96) diag_final_kernel(const double* __restrict__ chunks, const int* __restrict__ blk,
-                                                        int L, ObsTarget t) {
-    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nch = (diag_groups(blk[L]) + kDiagChunk - 1) / kDiagChunk;
-    double acc = 0.0;
-    for (int64_t c = lane; c < nch; c += 32) acc = __dadd_rn(acc, chunks[c * 3 + q]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-    if (lane != 0) return;
-    if (q == 0) {
-        if (t.norm) *t.norm = sqrt(acc);
-    } else if (q == 1) {
-        if (t.energy_re) *t.energy_re = acc;
-    } else {
-        if (t.energy_im) *t.energy_im = acc;
     }
 }
 
@@ -653,18 +658,19 @@ int launch_obs_t(const ModelDev& m, const uint64_t* keys, const int* blk, const 
             nb_s = grid_sg;
         }
     }
-    obs_final_kernel<<<sites ? 3 + 2 * m.L : 3, 256, 0, st>>>(m.L, nb_e, part_e, nb_s, part_s, out);
+    if (out.new_blk && !sites) return PACES_ERR_BADARG;  // step_end's block follows the sites'
+    obs_final_kernel<<<sites ? 3 + 2 * m.L + (out.new_blk ? 1 : 0) : 3, 256, 0, st>>>(m.L, nb_e, part_e, nb_s, part_s, out);
     return cudaGetLastError() == cudaSuccess ? PACES_OK : PACES_ERR_CUDA;
 }
 
 }  // namespace
 
-int launch_diag_final(const double* diag, const int* blk, int L, int64_t cap, const ObsTarget& out, cudaStream_t st) {
+int launch_diag_chunks(const double* diag, const int* blk, int L, int64_t cap, const double** out, cudaStream_t st) {
     if (!diag || cap < 0) return PACES_ERR_BADARG;
     double* chunks = const_cast<double*>(diag) + diag_groups(cap) * 3;
     const int64_t nch = diag_chunks(cap);
     diag_chunk_kernel<<<unsigned(nch > 0 ? nch : 1), 256, 0, st>>>(diag, chunks, blk, L);
-    diag_final_kernel<<<1, 96, 0, st>>>(chunks, blk, L, out);
+    *out = chunks;
     return cudaGetLastError() == cudaSuccess ? PACES_OK : PACES_ERR_CUDA;
 }
 

@@ -291,10 +291,10 @@ int taylor_max_grid(bool c64, int num_sms) {
 int launch_taylor(bool c64, const ModelDev& m, const int* blk, const int* nbr, int64_t nbr_cap,
                   const uint32_t* meta, const void* v_in, void* res, double dt, int m_star,
                   double tol, const TaylorWs& ws, const TaylorOut& out, int* status, int num_sms,
-                  int blocks_per_sm, int variant, cudaStream_t st) {
+                  int blocks_per_sm, int variant, cudaStream_t st, bool cleared) {
     if (m_star < 1 || variant < 0 || variant > 1) return PACES_ERR_BADARG;
     if (m.nhop > 1 && !m.xnbr) return PACES_ERR_BADARG;
-    if (cudaMemsetAsync(ws.barrier, 0, kTaylorBarrierBytes, st) != cudaSuccess) return PACES_ERR_CUDA;
+    if (!cleared && cudaMemsetAsync(ws.barrier, 0, kTaylorBarrierBytes, st) != cudaSuccess) return PACES_ERR_CUDA;
     const int geo = m.nhop > 1 ? m.hop_n[0] >> 1 : 0;
     const int occ = occupancy_any(c64, variant, geo);
     // a wave of blocks, or one block per 512 rows of room in a small problem (fewer blocks at the

@@ -633,7 +633,6 @@ int launch_truncate_t(const ModelDev& m, const uint64_t* x_keys, const int* x_bl
     constexpr bool kStore = WKS != WK;
     const void* src = kStore ? scratch : psi;
     const int g = grid_for(ws.cap, 1024, num_sms * 4);  // streaming passes of the tie shuffle
-    if (cudaMemsetAsync(ws.hist, 0, kTruncHistBytes, st) != cudaSuccess) return PACES_ERR_CUDA;
     {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid_for(ws.cap, kSelThreads * 2, max(num_sms / at_once, 1)));
@@ -688,7 +687,9 @@ int dispatch_prec(bool c64, const ModelDev& m, const uint64_t* x_keys, const int
 int launch_truncate(int nw, bool c64, const ModelDev& m, const uint64_t* x_keys, const int* x_blk,
                     const void* psi, const double* weights, void* scratch, int64_t maxstates, int shuffle, uint64_t seed,
                     uint64_t step, const TruncWs& ws, uint64_t* out_keys, int* out_blk, int64_t out_cap, float* out_w,
-                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, int at_once, cudaStream_t st) {
+                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, int at_once, cudaStream_t st,
+                    bool cleared) {
+    if (!cleared && cudaMemsetAsync(ws.hist, 0, kTruncHistBytes, st) != cudaSuccess) return PACES_ERR_CUDA;
 #define PACES_TRUNC_CASE(N)                                                                       \
     case N:                                                                                       \
         return dispatch_prec<N>(c64, m, x_keys, x_blk, psi, weights, scratch, maxstates, shuffle, seed, step, ws, \
