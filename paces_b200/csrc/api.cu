@@ -242,7 +242,7 @@ int64_t self_flag_cap(const paces_ctx* c, const Layout& l) {
 // The caller's Krylov workspace of the Lanczos step: order+1 vectors, two w buffers, the
 // per-block partial sums and the barrier words.
 struct KrylovLayout {
-    size_t u, w0, w1, partials, barrier, total;
+    size_t u, partials, barrier, total;
     int max_grid;
 };
 
@@ -256,9 +256,7 @@ KrylovLayout krylov_layout(const paces_ctx* c, int64_t cap, int order) {
     };
     const size_t cs = c->precision == PACES_C64 ? 8 : 16;
     k.max_grid = lanczos_max_grid(c->num_sms);
-    k.u = take(size_t(order + 1) * size_t(cap) * cs);
-    k.w0 = take(size_t(cap) * cs);
-    k.w1 = take(size_t(cap) * cs);
+    k.u = take(size_t(order) * size_t(cap) * cs);
     k.partials = take(size_t(2) * k.max_grid * 4 * 8);
     k.barrier = take(16);
     k.total = off;
@@ -279,8 +277,6 @@ LanczosWs lanczos_ws(const paces_ctx* c, void* krylov, int64_t cap, int order) {
     const KrylovLayout k = krylov_layout(c, cap, order);
     LanczosWs w;
     w.u = at<void>(krylov, k.u);
-    w.w0 = at<void>(krylov, k.w0);
-    w.w1 = at<void>(krylov, k.w1);
     w.partials = at<double>(krylov, k.partials);
     w.barrier = at<unsigned>(krylov, k.barrier);
     w.cap = cap;

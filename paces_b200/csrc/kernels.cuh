@@ -112,9 +112,7 @@ __device__ __forceinline__ void diag_group(double* __restrict__ diag, int64_t g,
 // ---- Lanczos ----------------------------------------------------------------------------
 constexpr int kMaxLanczosOrder = PACES_MAX_LANCZOS_ORDER;
 struct LanczosWs {
-    void* u;             // [order+1][cap] complex: the Krylov vectors q_i (columns of V)
-    void* w0;            // [cap] complex: the recurrence's w, double-buffered
-    void* w1;
+    void* u;             // [order][cap] complex: the unnormalised Krylov columns 1 .. order
     double* partials;    // [2][max_grid][4]
     unsigned* barrier;   // [2]
     int64_t cap;         // rows of each vector
