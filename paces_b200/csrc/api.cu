@@ -86,7 +86,7 @@ struct Layout {
     size_t t_hist, t_cand, t_cand_idx, t_sel, t_sum, t_chunk;
     size_t r_tile_off, r_counters, r_split;
     int r_tiles;
-    size_t v_V, v_TA, v_TB, v_partials, v_bar;
+    size_t v_V, v_TA, v_TB, v_bar;
     size_t o_partials, o_out;
     size_t aw, keep;  // kept amplitudes of the truncation, proposal keep mask [kRuns][cap]
     size_t maps_e, keysN, blkN, n2b;  // split expansion: its maps, the new part, new part -> output
@@ -133,7 +133,6 @@ Layout make_layout(const paces_ctx* c, int64_t cap) {
     l.v_V = take(ucap * cs);
     l.v_TA = take(ucap * cs);
     l.v_TB = take(ucap * cs);
-    l.v_partials = take(size_t(2) * c->taylor_grid * 4 * 8);
     l.v_bar = take(kTaylorBarrierBytes);
     l.o_partials = take(size_t(obs_max_grid(c->num_sms)) * (4 + 2 * L) * 8);
     l.o_out = take(size_t(3 + 2 * L) * 8);
@@ -219,7 +218,6 @@ TaylorWs taylor_ws(const paces_ctx* c, const Layout& l, void* ws) {
     TaylorWs w;
     w.ta = at<void>(ws, l.v_TA);
     w.tb = at<void>(ws, l.v_TB);
-    w.partials = at<double>(ws, l.v_partials);
     w.barrier = at<unsigned>(ws, l.v_bar);
     w.maxima = at<unsigned long long>(ws, l.v_bar + kTaylorMaximaOffset);
     w.wait_ns = c->test_wait_ns ? c->test_wait_ns : kWaitLimitNs;
@@ -1155,7 +1153,7 @@ int paces_expm_scaled(paces_ctx* c, const paces_basis* b, const paces_hmat* h, c
     }
     PACES_CHECK_LAUNCH(c, launch_expm_scaled(c->precision == PACES_C64, with_h(c, h), b->blk, h->nbr, h->meta, psi_in, psi_out,
                                              t, shift, m_star, stages, tol, eta_re, eta_im, taylor_ws(c, l, ws), o,
-                                             c->d_status, c->num_sms, c->taylor_grid,
+                                             c->d_status, c->num_sms,
                                              reinterpret_cast<cudaStream_t>(stream)),
                        "expm_scaled");
     return PACES_OK;

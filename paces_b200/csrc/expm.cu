@@ -12,35 +12,20 @@
 // B200 design: the norms are two deterministic reductions over the neighbour table; the
 // whole series -- every term of every stage and the stage-end phase factors -- is one
 // persistent cooperative launch with a bounded grid barrier between sweeps, as in the
-// plain Taylor kernel.  Each stage's first term reads a copy of F (made during the
+// plain Taylor kernel.  A sweep is short (190K rows: a few microseconds), so what closes it counts:
+// its maxima go through grid_max's atomics instead of a partial per block that every block reads
+// back, and a thread's two rows have their loads in flight together (a scaled step of 50K kept
+// states with both and the norms' reduction below: 688 -> 619 us).  Each stage's first term reads a copy of F (made during the
 // stage-end sweep), so no sweep gathers from a vector it is writing.
-#include "grid.cuh"
-#include "hrow.cuh"
 #include "kernels.cuh"
+#include "taylor_row.cuh"
 
 namespace paces {
 
 namespace {
 
-constexpr int kEThreads = 256;
-constexpr int kEWarps = kEThreads / 32;
-
-__device__ void block_max4(double v[4], double (*red)[kEWarps], double* out) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] = fmax(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-        if (lane == 0) red[k][wid] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < 4) {
-        double r = 0.0;
-        for (int w = 0; w < kEWarps; ++w) r = fmax(r, red[threadIdx.x][w]);
-        out[threadIdx.x] = r;
-    }
-    __syncthreads();
-}
+constexpr int kEThreads = kStreamThreads;
+constexpr int kEWarps = kStreamWarps;
 
 // Per-block partials of the trace (sum of diagonal elements, [0]) and of the largest row
 // 1-norm of H - shift I ([1]; only when shift is given).
@@ -93,14 +78,31 @@ hnorm_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ nb
 }
 
 // Fixed-order reduction of the partials: out[0] = trace, out[1] = max row 1-norm,
-// out[2] = trace / n.
-__global__ void hnorm_final_kernel(const int* __restrict__ blk, int L, const double* __restrict__ part, int nparts,
-                                   double* __restrict__ out) {
-    if (threadIdx.x != 0) return;
+// out[2] = trace / n.  One block: its threads' strided sums, the warps' butterflies, the warps in
+// order.  (One thread over all partials took 24 us, twice a step.)
+__global__ void __launch_bounds__(kEThreads) hnorm_final_kernel(const int* __restrict__ blk, int L,
+                                                                const double* __restrict__ part, int nparts,
+                                                                double* __restrict__ out) {
+    __shared__ double s_sum[kEWarps], s_max[kEWarps];
     double a = 0.0, b = 0.0;
-    for (int i = 0; i < nparts; ++i) {
+    for (int i = threadIdx.x; i < nparts; i += kEThreads) {
         a += part[2 * i];
         b = fmax(b, part[2 * i + 1]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s_sum[threadIdx.x >> 5] = a;
+        s_max[threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < kEWarps; ++w) {
+        a += s_sum[w];
+        b = fmax(b, s_max[w]);
     }
     const int64_t S = blk[L];
     out[0] = a;
@@ -109,7 +111,7 @@ __global__ void hnorm_final_kernel(const int* __restrict__ blk, int L, const dou
 }
 
 template <bool C64>
-__global__ void __launch_bounds__(kEThreads, C64 ? 4 : 3)
+__global__ void __launch_bounds__(kEThreads, C64 ? 3 : 2)
 expm_scaled_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ nbr,
                    const uint32_t* __restrict__ meta, const void* v_in, void* res_out, TaylorWs ws, double t,
                    double shift, int m_star, int stages, double tol, double eta_re, double eta_im, TaylorOut out,
@@ -118,7 +120,7 @@ expm_scaled_kernel(ModelDev m, const int* __restrict__ blk, const int* __restric
     using R = typename std::conditional<C64, float, double>::type;
     __shared__ R s_sq[260];
     __shared__ double s_red[4][kEWarps];
-    __shared__ double s_fin[4];
+    __shared__ double s_fin[5];
     for (int k = threadIdx.x; k < 260; k += kEThreads) s_sq[k] = R(__dmul_rn(sqrt(double(k)), m.g));
     __syncthreads();
     const int64_t S = blk[m.L];
@@ -144,56 +146,60 @@ expm_scaled_kernel(ModelDev m, const int* __restrict__ blk, const int* __restric
             const C* rin = (st == 0 && j == 0) ? v : res;
             const double cd = t / (double(stages) * double(j + 1));
             const R c = R(cd);
-            double mx[4] = {0.0, 0.0, 0.0, 0.0};  // |B|, |F|, |B at stage start|, non-finite
-            for (int64_t r = r0; r < S; r += stride) {
-                const uint32_t mm = __ldg(meta + r);
+            SweepMax<R> mx{R(0), R(0), R(0), R(0)};  // |B|^2, |F|^2, |B at stage start|^2
+            // y = (H - shift) B of one row, from its own element x
+            auto shifted = [&](int64_t r, const C& x) -> C {
                 C y;
-                const C xr = __ldcg(src + r);
                 if constexpr (C64) {
-                    y = h_row_c64_any(m, s_sq, J, r, load_nbr(nbr, r), mm, __ldcg(src + r), src);
-                    y.x = fmaf(-sh, xr.x, y.x);
-                    y.y = fmaf(-sh, xr.y, y.y);
+                    y = h_row_c64_any(m, s_sq, J, r, load_nbr(nbr, r), __ldg(meta + r), x, src);
+                    y.x = fmaf(-sh, x.x, y.x);
+                    y.y = fmaf(-sh, x.y, y.y);
                 } else {
-                    y = h_row_c128_any(m, s_sq, r, load_nbr(nbr, r), mm, __ldcg(src + r), src);
-                    y.x = __dsub_rn(y.x, __dmul_rn(sh, xr.x));
-                    y.y = __dsub_rn(y.y, __dmul_rn(sh, xr.y));
+                    y = h_row_c128_any(m, s_sq, r, load_nbr(nbr, r), __ldg(meta + r), x, src);
+                    y.x = __dsub_rn(y.x, __dmul_rn(sh, x.x));
+                    y.y = __dsub_rn(y.y, __dmul_rn(sh, x.y));
                 }
-                // B = c * i * y
+                return y;
+            };
+            // B <- c i y, F <- F + B
+            auto finish = [&](int64_t r, const C& x, const C& y, const C& a) {
                 C b, f;
-                const C a = rin[r];
                 if constexpr (C64) {
                     b = make_float2(-(c * y.y), c * y.x);
                     f = make_float2(a.x + b.x, a.y + b.y);
-                    mx[0] = fmax(mx[0], double(fmaf(b.x, b.x, b.y * b.y)));
-                    mx[1] = fmax(mx[1], double(fmaf(f.x, f.x, f.y * f.y)));
-                    if (j == 0) mx[2] = fmax(mx[2], double(fmaf(xr.x, xr.x, xr.y * xr.y)));
+                    mx.term = fmax(mx.term, fmaf(b.x, b.x, b.y * b.y));
+                    mx.res = fmax(mx.res, fmaf(f.x, f.x, f.y * f.y));
+                    if (j == 0) mx.v = fmax(mx.v, fmaf(x.x, x.x, x.y * x.y));
                 } else {
                     b = make_double2(-__dmul_rn(cd, y.y), __dmul_rn(cd, y.x));
                     f = make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
-                    mx[0] = fmax(mx[0], fma(b.x, b.x, b.y * b.y));
-                    mx[1] = fmax(mx[1], fma(f.x, f.x, f.y * f.y));
-                    if (j == 0) mx[2] = fmax(mx[2], fma(xr.x, xr.x, xr.y * xr.y));
+                    mx.term = fmax(mx.term, fma(b.x, b.x, b.y * b.y));
+                    mx.res = fmax(mx.res, fma(f.x, f.x, f.y * f.y));
+                    if (j == 0) mx.v = fmax(mx.v, fma(x.x, x.x, x.y * x.y));
                 }
-                if (!(isfinite(double(f.x)) && isfinite(double(f.y)))) mx[3] = 1.0;
+                note(mx.nan, f);
                 dst[r] = b;
                 res[r] = f;
+            };
+            // two rows a grid stride apart, their loads in flight together
+            int64_t r = r0;
+            for (; r + stride < S; r += 2 * stride) {
+                const C x0 = __ldcg(src + r), x1 = __ldcg(src + r + stride);
+                const C a0 = rin[r], a1 = rin[r + stride];
+                const C y0 = shifted(r, x0), y1 = shifted(r + stride, x1);
+                finish(r, x0, y0, a0);
+                finish(r + stride, x1, y1, a1);
             }
-            block_max4(mx, s_red, s_fin);
-            if (threadIdx.x == 0) {
-                double* pp = ws.partials + (size_t((final_m & 1) * nblocks) + blockIdx.x) * 4;
-                for (int k = 0; k < 4; ++k) pp[k] = s_fin[k];
+            if (r < S) {
+                const C x0 = __ldcg(src + r), a0 = rin[r];
+                finish(r, x0, shifted(r, x0), a0);
             }
-            if (!grid_barrier(ws.barrier, nblocks, gen, status, ws.wait_ns, int(blockIdx.x) == ws.skip_block)) {
+            if (!grid_max(mx, ws.maxima + (final_m % 3) * 4, s_red, s_fin, ws, gen, status)) {
                 stop = true;
                 break;
             }
-            double g4[4] = {0.0, 0.0, 0.0, 0.0};
-            for (unsigned bb = threadIdx.x; bb < nblocks; bb += kEThreads) {
-                const double* pp = ws.partials + (size_t((final_m & 1) * nblocks) + bb) * 4;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) g4[k] = fmax(g4[k], __ldcg(pp + k));
-            }
-            block_max4(g4, s_red, s_fin);
+            // the buffer that the sweep after next folds into
+            if (blockIdx.x == 0 && threadIdx.x < 4) ws.maxima[((final_m + 2) % 3) * 4 + threadIdx.x] = 0ull;
             ++final_m;
             if (s_fin[3] != 0.0) {
                 if (blockIdx.x == 0 && threadIdx.x == 0) raise_status(status, PACES_ERR_NONFINITE);
@@ -251,18 +257,17 @@ int expm_occupancy() {
 int launch_hnorms(const ModelDev& m, const int* blk, const int* nbr, const uint32_t* meta, const double* shift,
                   double* part, int nparts, double* out, cudaStream_t st) {
     hnorm_kernel<<<nparts, kEThreads, 0, st>>>(m, blk, nbr, meta, shift, part);
-    hnorm_final_kernel<<<1, 32, 0, st>>>(blk, m.L, part, nparts, out);
+    hnorm_final_kernel<<<1, kEThreads, 0, st>>>(blk, m.L, part, nparts, out);
     return cudaGetLastError() == cudaSuccess ? PACES_OK : PACES_ERR_CUDA;
 }
 
 int launch_expm_scaled(bool c64, const ModelDev& m, const int* blk, const int* nbr, const uint32_t* meta,
                        const void* v_in, void* res, double t, double shift, int m_star, int stages, double tol,
                        double eta_re, double eta_im, const TaylorWs& ws, const TaylorOut& out, int* status,
-                       int num_sms, int max_grid, cudaStream_t st) {
+                       int num_sms, cudaStream_t st) {
     if (m_star < 0 || stages < 1) return PACES_ERR_BADARG;
-    if (cudaMemsetAsync(ws.barrier, 0, 2 * sizeof(unsigned), st) != cudaSuccess) return PACES_ERR_CUDA;
-    int grid = num_sms * (c64 ? expm_occupancy<true>() : expm_occupancy<false>());
-    if (grid > max_grid) grid = max_grid;  // the partials buffer holds max_grid blocks
+    if (cudaMemsetAsync(ws.barrier, 0, kTaylorBarrierBytes, st) != cudaSuccess) return PACES_ERR_CUDA;
+    const int grid = num_sms * (c64 ? expm_occupancy<true>() : expm_occupancy<false>());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kEThreads);

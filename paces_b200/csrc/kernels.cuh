@@ -47,7 +47,6 @@ struct TaylorOut {
 struct TaylorWs {
     void* ta;            // [cap] complex
     void* tb;            // [cap] complex
-    double* partials;    // [2][max_grid][4]
     unsigned* barrier;   // grid_barrier's counter, and maxima behind it: kTaylorBarrierBytes, zeroed per launch
     unsigned long long* maxima;  // [3][4] a sweep's maxima (fp64 bit patterns), the buffers in rotation
     uint64_t wait_ns;    // grid-barrier wait limit (kWaitLimitNs unless a test shortens it)
@@ -147,7 +146,7 @@ int launch_hnorms(const ModelDev& m, const int* blk, const int* nbr, const uint3
 int launch_expm_scaled(bool c64, const ModelDev& m, const int* blk, const int* nbr, const uint32_t* meta,
                        const void* v_in, void* res, double t, double shift, int m_star, int stages, double tol,
                        double eta_re, double eta_im, const TaylorWs& ws, const TaylorOut& out, int* status,
-                       int num_sms, int max_grid, cudaStream_t st);
+                       int num_sms, cudaStream_t st);
 
 // ---- look-ahead truncation weights (lookahead.cu) -------------------------------------------
 // w[r] for every row of the basis (blk[L] rows): kind is PACES_WEIGHT_COHERENCE, _NORM or

@@ -46,37 +46,6 @@ namespace {
 constexpr int kTThreads = kStreamThreads;
 constexpr int kTWarps = kTThreads / 32;
 
-// Fold the block's maxima into g[0..3] (fp64 bit patterns; atomicMax is exact and order-free),
-// pass the grid barrier and read the grid's maxima into fin[0..3] (shared; fin[4] is the
-// barrier's success).  false on a timeout.
-template <typename R>
-__device__ bool grid_max(const SweepMax<R>& mx, unsigned long long* g, double (*red)[kTWarps], double* fin,
-                         const TaylorWs& ws, unsigned& gen, int* status) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const R a = warp_max(mx.term), b = warp_max(mx.res), c = warp_max(mx.v);
-    const bool bad = __any_sync(0xffffffffu, mx.nan != R(0));
-    if (lane == 0) {
-        red[0][wid] = double(a);
-        red[1][wid] = double(b);
-        red[2][wid] = double(c);
-        red[3][wid] = bad ? 1.0 : 0.0;
-    }
-    __syncthreads();
-    if (wid == 0) {
-        double r = 0.0;
-        if (lane < 4)
-            for (int w = 0; w < kTWarps; ++w) r = fmax(r, red[lane][w]);
-        if (r > 0.0) atomicMax(g + lane, static_cast<unsigned long long>(__double_as_longlong(r)));
-        __syncwarp();
-        const bool ok = grid_barrier_warp(ws.barrier, gridDim.x, gen, status, ws.wait_ns, int(blockIdx.x) == ws.skip_block);
-        if (lane < 4) fin[lane] = __longlong_as_double((long long)__ldcg(g + lane));
-        if (lane == 4) fin[4] = ok ? 1.0 : 0.0;
-    }
-    ++gen;
-    __syncthreads();
-    return fin[4] != 0.0;
-}
-
 // GEO: 0 the chain, otherwise the dimensions of a lattice with several hopping channels (h_row_*_geo).
 template <bool C64, bool STREAM, int GEO>
 __global__ void __launch_bounds__(kTThreads, STREAM ? (C64 ? 3 : 2) : (C64 ? 4 : 3))

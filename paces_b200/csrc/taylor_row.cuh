@@ -1,12 +1,14 @@
 // Row arithmetic and maxima shared by the Taylor kernels (single, batched).
 #pragma once
 
+#include "grid.cuh"
 #include "hrow.cuh"
 #include "kernels.cuh"
 
 namespace paces {
 
 constexpr int kStreamThreads = 256;  // threads per block of the kernels that stream rows
+constexpr int kStreamWarps = kStreamThreads / 32;
 
 // Largest of a warp's non-negative values (their bit patterns order like the values).
 __device__ __forceinline__ float warp_max(float v) {
@@ -24,6 +26,37 @@ struct SweepMax {
     R term, res, v;
     R nan;  // 0, or a NaN once an element was not finite
 };
+
+// Fold the block's maxima into g[0..3] (fp64 bit patterns; atomicMax is exact and order-free),
+// pass the grid barrier and read the grid's maxima into fin[0..3] (shared; fin[4] is the
+// barrier's success).  false on a timeout.
+template <typename R>
+__device__ __forceinline__ bool grid_max(const SweepMax<R>& mx, unsigned long long* g, double (*red)[kStreamWarps], double* fin,
+                         const TaylorWs& ws, unsigned& gen, int* status) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const R a = warp_max(mx.term), b = warp_max(mx.res), c = warp_max(mx.v);
+    const bool bad = __any_sync(0xffffffffu, mx.nan != R(0));
+    if (lane == 0) {
+        red[0][wid] = double(a);
+        red[1][wid] = double(b);
+        red[2][wid] = double(c);
+        red[3][wid] = bad ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    if (wid == 0) {
+        double r = 0.0;
+        if (lane < 4)
+            for (int w = 0; w < kStreamWarps; ++w) r = fmax(r, red[lane][w]);
+        if (r > 0.0) atomicMax(g + lane, static_cast<unsigned long long>(__double_as_longlong(r)));
+        __syncwarp();
+        const bool ok = grid_barrier_warp(ws.barrier, gridDim.x, gen, status, ws.wait_ns, int(blockIdx.x) == ws.skip_block);
+        if (lane < 4) fin[lane] = __longlong_as_double((long long)__ldcg(g + lane));
+        if (lane == 4) fin[4] = ok ? 1.0 : 0.0;
+    }
+    ++gen;
+    __syncthreads();
+    return fin[4] != 0.0;
+}
 
 // Separate roundings (no contraction into an FMA), so
 // that every kernel and schedule that runs these rows -- direct, bulk, batched -- rounds alike.
