@@ -246,19 +246,23 @@ def max_over_ranks(value, dist, device="cuda"):
     return float(t.item())
 
 
-def taylor_bytes_per_term(rec, cs):
-    """Algorithmic bytes of one Taylor term on S rows: neighbour table (16 B), row metadata
-    (4 B), previous term read once, result read and written, new term written (4*cs)."""
-    return rec.n_states * (16 + 4 + 4 * cs)
+def taylor_bytes(rec, cs):
+    """Algorithmic bytes of a Taylor series of final_m + 1 terms on S rows.  Every sweep reads the
+    neighbour table (16 B), the row metadata (4 B) and the previous term and writes the new one
+    (2*cs); every second one also reads and writes the sum, adding two terms (2*cs); a last
+    odd term is added by a pass of its own (3*cs)."""
+    n = rec.final_m + 1
+    return rec.n_states * (n * (16 + 4 + 2 * cs) + (n // 2) * 2 * cs + (n % 2) * 3 * cs)
 
 
 def lanczos_bytes(rec, cs, order):
     """Algorithmic bytes of one Lanczos propagation on S rows with order + 1 vectors: the norm
-    pass (S*cs); per vector sweep A (table 16 B, metadata 4 B, the gathered source, q_{i-1}
-    read, q_i and w written: 4*cs) and, but for the last vector, sweep B (w read and written,
-    q_i read: 3*cs); the final combination (order + 1 vectors read, the result written)."""
+    pass (S*cs); per vector sweep A (table 16 B, metadata 4 B, the gathered column, the column
+    before it (not for the first) read, the next written (not for the last): 3*cs) and, but for
+    the last vector, sweep B (the next column read and written, this one read: 3*cs); the final
+    combination (order + 1 columns read, the result written)."""
     k = order + 1
-    return rec.n_states * (cs + k * (20 + 4 * cs) + (k - 1) * 3 * cs + (k + 1) * cs)
+    return rec.n_states * (cs + k * (20 + 3 * cs) - 2 * cs + (k - 1) * 3 * cs + (k + 1) * cs)
 
 
 def step_bytes(rec, cs, nw, es):
@@ -271,7 +275,7 @@ def step_bytes(rec, cs, nw, es):
     expand = es * (M * kb + B * kb)                  # read the basis once, write the enlarged basis
     assemble = B * kb + S * kb + S * (16 + 4) + 5 * B * 4 + B * 32   # keys in/out, H table, maps, fill
     remap = 2 * S * kb + 2 * S * cs
-    taylor = (rec.final_m + 1) * S * (16 + 4 + 4 * cs)
+    taylor = taylor_bytes(rec, cs)
     obs = 2 * S * (cs + 4 + 16) + S * kb
     return truncate + expand + assemble + remap + taylor + obs
 
@@ -471,7 +475,7 @@ def run_ours(a):
     if a.lanczos_order:
         taylor_alg = statistics.mean(lanczos_bytes(r, cs, a.lanczos_order) for r in prof_recs)
     else:
-        taylor_alg = statistics.mean(taylor_bytes_per_term(r, cs) * (r.final_m + 1) for r in prof_recs)
+        taylor_alg = statistics.mean(taylor_bytes(r, cs) for r in prof_recs)
     achieved = taylor_alg / (taylor_ms / 1e3) / 1e9
     peak, peak_kind = read_peaks()
     per_row_term = read_profile_traffic(a.precision)
@@ -888,7 +892,7 @@ def run_batched(a):
     n = len(trajs)
     value = n * a.steps * world / (ms / 1e3)
     taylor_ms = phase["taylor"] / n_prof
-    taylor_alg = statistics.mean(sum(taylor_bytes_per_term(r, cs) * (r.final_m + 1) for r in rr) for rr in prof)
+    taylor_alg = statistics.mean(sum(taylor_bytes(r, cs) for r in rr) for rr in prof)
     achieved = taylor_alg / (taylor_ms / 1e3) / 1e9
     peak, peak_kind = read_peaks()
     states = statistics.mean(sum(r.n_states for r in rr) for rr in rounds)
@@ -1003,7 +1007,7 @@ def run_learned(a):
     cs = 8
     taylor_ms = stage["taylor"] / max(nprof, 1)
     win = recs[lf + 1:]
-    taylor_alg = statistics.mean(taylor_bytes_per_term(r, cs) * (r.final_m + 1) for r in win)
+    taylor_alg = statistics.mean(taylor_bytes(r, cs) for r in win)
     peak, peak_kind = read_peaks()
     achieved = taylor_alg / (taylor_ms / 1e3) / 1e9 if taylor_ms > 0 else None
     if rank == 0:
@@ -1160,7 +1164,7 @@ def run_longchain(a):
     n = len(seeds)
     value = n * a.steps * world / (ms / 1e3)
     taylor_ms = phase["taylor"] / n_prof
-    taylor_alg = statistics.mean(sum(taylor_bytes_per_term(r, cs) * (r.final_m + 1) for r in rr) for rr in prof)
+    taylor_alg = statistics.mean(sum(taylor_bytes(r, cs) for r in rr) for rr in prof)
     achieved = taylor_alg / (taylor_ms / 1e3) / 1e9
     peak, peak_kind = read_peaks()
     if rank == 0:

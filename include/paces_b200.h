@@ -286,7 +286,7 @@ typedef struct paces_tuning {
     int32_t merge_stride_min;          /* read only */
     int32_t merge_stride_max;          /* read only */
     int32_t taylor_blocks_per_sm_max;  /* read only */
-    int32_t taylor_variant;            /* 0: rows read directly; 1: 512-row chunks prefetched by bulk copies */
+    int32_t taylor_variant;            /* 0: rows read directly; 1: rows streamed through registers */
     int32_t assemble_stride;           /* the assembly's stride, same range; 0 on set: merge_stride */
     int32_t reserved[1];
 } paces_tuning;

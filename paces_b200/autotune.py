@@ -7,7 +7,7 @@ arithmetic and ordering are fixed by the data, not by the tiling):
   and one for the assembly: larger tiles spend less on splitters and look-back, smaller ones
   fit more blocks per SM;
 * the persistent Taylor kernel's blocks per SM (its grid) and its row schedule (rows read
-  directly, or 512-row chunks prefetched into shared memory by bulk TMA copies).
+  directly, or streamed through registers with the next rows on their way).
 
 `tune(trajectory, dt)` times candidates on the live workload -- eager steps with the
 library's stage events -- and keeps, shape by shape, the fastest (the expansion stride by
@@ -32,7 +32,7 @@ from . import _native as nat
 CACHE_PATH = os.environ.get("PACES_TUNE_CACHE",
                             os.path.join(os.path.expanduser("~"), ".cache", "paces_b200", "tuning.json"))
 _memory: dict = {}
-VARIANTS = [0, 1]  # Taylor row schedules: direct, bulk-prefetched
+VARIANTS = [0, 1]  # Taylor row schedules: direct, streamed
 SHAPES = ("merge_stride", "taylor_blocks_per_sm", "taylor_variant", "assemble_stride")
 
 

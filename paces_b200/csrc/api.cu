@@ -20,7 +20,7 @@ struct paces_ctx {
     int merge_stride;     // tuning: elements per splitter of the expansions' merge tiles
     int assemble_stride;  // tuning: the same for the assembly
     int taylor_bps;    // tuning: Taylor blocks per SM (0 = as many as fit)
-    int taylor_variant;  // tuning: 0 direct rows, 1 bulk-prefetched chunks
+    int taylor_variant;  // tuning: 0 direct rows, 1 streamed rows
     int* d_status;  // device status word for the stage entry points (start of the constants block)
     double* d_site_eps;  // [kMaxSites] per-site energies, device copy (batched Taylor)
     double* d_sq;        // [kSqrtTable] sqrt(k) * g
@@ -1454,8 +1454,8 @@ int paces_batch_step(paces_batch* b, const paces_batch_item* items, int32_t n, p
     mark(1);
     // 2. the Taylor series.  Batches of large trajectories (every evolving one with room for at
     //    least kBatchSingleCap states) run them one after the other through the single-trajectory
-    //    kernel, whose bulk-copy schedule streams long row ranges faster (0.85 against 0.61 of
-    //    HBM on 64M-row trajectories); otherwise one persistent launch serves all.  Both give
+    //    kernel (0.85 against 0.61 of HBM on 64M-row trajectories, measured before both kernels
+    //    streamed rows through registers); otherwise one persistent launch serves all.  Both give
     //    the same results.  Test hooks on the batch keep the batched launch.
     bool per_item = n_evolve > 0 && b->test_wait_ns == 0 && b->test_skip_block < 0;
     for (int i = 0; i < n && per_item; ++i)

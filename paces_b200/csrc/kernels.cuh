@@ -61,8 +61,9 @@ int taylor_max_grid(bool c64, int num_sms);
 // The first sweep of the series forms (H v)_r for every row, so the post-adaptation norm and
 // energy <v|H|v> come out of it: each warp folds the rows of one 64-row group (rows 64 g + l and
 // 64 g + 32 + l on lane l, in every kernel and schedule: the lane adds its two rows, then a fixed
-// butterfly), and diag_final sums the groups in a fixed order.  The result depends on the rows
-// only -- not on the grid, the row schedule or whether the trajectory runs alone or in a batch.
+// butterfly), and diag_chunk_kernel and step_end sum the groups in a fixed order.  The result
+// depends on the rows only -- not on the grid, the row schedule or whether the trajectory runs
+// alone or in a batch.
 constexpr int kDiagGroup = 64;
 constexpr int kDiagChunk = 2048;  // groups per block of the first reduction
 __host__ __device__ inline int64_t diag_groups(int64_t rows) { return (rows + kDiagGroup - 1) / kDiagGroup; }
@@ -131,7 +132,7 @@ int launch_lanczos(bool c64, const ModelDev& m, const int* blk, const int* nbr, 
                    const void* v_in, void* res, double dt, int order, const LanczosWs& ws, const TaylorOut& out,
                    int* status, int num_sms, cudaStream_t st);
 // blocks_per_sm: 0 = as many as fit (the grid never exceeds taylor_max_grid);
-// variant: 0 = direct grid-stride rows, 1 = chunks prefetched by bulk TMA copies
+// variant: 0 = direct grid-stride rows, 1 = rows streamed through registers, the sum a term behind
 int launch_taylor(bool c64, const ModelDev& m, const int* blk, const int* nbr, int64_t nbr_cap,
                   const uint32_t* meta, const void* v_in, void* res, double dt, int m_star,
                   double tol, const TaylorWs& ws, const TaylorOut& out, int* status, int num_sms,

@@ -59,7 +59,7 @@ __device__ __forceinline__ bool grid_max(const SweepMax<R>& mx, unsigned long lo
 }
 
 // Separate roundings (no contraction into an FMA), so
-// that every kernel and schedule that runs these rows -- direct, bulk, batched -- rounds alike.
+// that every kernel and schedule that runs these rows -- direct, streamed, batched -- rounds alike.
 __device__ __forceinline__ float sq_abs(const float2& z) { return fmaf(z.x, z.x, __fmul_rn(z.y, z.y)); }
 __device__ __forceinline__ double sq_abs(const double2& z) { return fma(z.x, z.x, __dmul_rn(z.y, z.y)); }
 __device__ __forceinline__ float2 add_c(const float2& a, const float2& t) {
