@@ -322,6 +322,18 @@ class Engine:
                                         _stream(self.device)), self.ctx, "hnorms")
         return [float(x) for x in out.cpu().tolist()]
 
+    def shifted_norm(self, b: DevBasis, h: DevHMat):
+        """(trace / n, largest row 1-norm of H - (trace / n) I): hnorms twice, the second one's
+        shift taken on the device, one read of both (a read between them cost a round trip)."""
+        out = torch.empty(6, dtype=torch.float64, device=self.device)
+        ws, nb = self.workspace()
+        bc, hc, st = b.c(), h.c(), _stream(self.device)
+        for sh, o in ((None, out[:3]), (out[2:3], out[3:])):
+            nat.check(self.lib.paces_hnorms(self.ctx, ctypes.byref(bc), ctypes.byref(hc), _ptr(sh), _ptr(o), ws, nb, st),
+                      self.ctx, "hnorms")
+        x = out.cpu().tolist()
+        return float(x[2]), float(x[4])
+
     def expm_scaled(self, b: DevBasis, h: DevHMat, psi_in, psi_out, t, shift, m_star, stages, eta, tol=None):
         """psi_out = exp(t * 1j (H - shift I)) psi_in in `stages` stages of at most m_star terms,
         times eta after each stage.  Returns [converged, final_m, c1 + c2, term ratio]."""
@@ -664,8 +676,7 @@ class Trajectory:
         capacity.  Returns [converged, final_m, c1_plus_c2, term_ratio]."""
         from . import expm
         e, b, h = self.eng, self.basis, self.h
-        _, _, dbar = e.hnorms(b, h)
-        _, a1, _ = e.hnorms(b, h, shift=dbar)
+        dbar, a1 = e.shifted_norm(b, h)
         ta = abs(t)  # the choice depends on |t| ||A||; a negative t propagates backwards
         m, s = expm.choose(ta * a1, d=lambda p: self._norm_power(ta, dbar, p))
         eta = np.exp(t * 1j * dbar / s)
