@@ -222,9 +222,10 @@ __device__ __forceinline__ void pick_bin(const unsigned (&hb)[PER], long long ne
 //    from the grid's histogram itself.  The first pass bins 64 binades below 2 by 6 mantissa
 //    bits (what lies below or above goes to its end bins): exponents alone put most states
 //    into a few bins, whose atomics collide.
+//    An end bin is no power of two wide, so the next pass's last bin may be cut short.
 //  * Once the chosen bin holds at most kSelCand states (two passes leave a few of millions;
-//    all bits take up to 6 passes), one more pass lists the bin's states and every block
-//    settles the remaining bits among them.
+//    all bits take 5 passes, 7 from an end bin of the first), one more pass lists the bin's
+//    states and every block settles the remaining bits among them.
 //  * That pass also counts the states above the bin per chunk of the compaction; with the
 //    listed states added and the blocks' totals exchanged, the counts become every chunk's
 //    prefix (states above the threshold | tied states << 31), so the compaction's warps need
@@ -306,8 +307,9 @@ trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restr
         }
         const unsigned long long bin = (unsigned long long)s_pick[0];
         if (round > 0) {
+            // the last bin ends with the range: what lies past it was counted as above before
+            width = min(1ull << shift, width - (bin << shift));
             lo += bin << shift;
-            width = 1ull << shift;
         } else {
             lo = bin == 0 ? 0ull : kFirstBase + (bin << shift);
             width = bin == 0 ? kFirstBase + (1ull << shift) : (bin == 4095 ? 0ull - lo : 1ull << shift);
@@ -377,8 +379,9 @@ trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restr
                 if (blockIdx.x == 0 && tid == 0) raise_status(status, PACES_ERR_BADARG);
                 return;
             }
-            lo += (unsigned long long)s_pick[0] << shift;
-            width = 1ull << shift;
+            const unsigned long long off = (unsigned long long)s_pick[0] << shift;
+            width = min(1ull << shift, width - off);  // as above
+            lo += off;
             need -= s_pick[1];
             ties = s_pick[2];
         }
