@@ -13,7 +13,9 @@ namespace paces {
 // other block's wait runs out.
 
 // By all lanes of one warp, for a block whose other warps' accesses this warp has synchronised
-// with; the caller advances `gen` and synchronises the block afterwards.
+// with; the caller advances `gen` and synchronises the block afterwards.  Lane 0 acquires the
+// other blocks' writes; the warp barrier behind its wait (a shuffle orders no memory) lets every
+// lane of the warp read them, as the callers that fold the blocks' values do.
 __device__ __forceinline__ bool grid_barrier_warp(unsigned* bar, unsigned nblocks, unsigned gen, int* status,
                                                   uint64_t limit_ns = kWaitLimitNs, bool skip = false) {
     int ok = 1;
@@ -37,6 +39,7 @@ __device__ __forceinline__ bool grid_barrier_warp(unsigned* bar, unsigned nblock
             }
         }
     }
+    __syncwarp();
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
