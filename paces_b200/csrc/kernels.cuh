@@ -157,6 +157,7 @@ int launch_lookahead(bool c64, const ModelDev& m, const int* blk, const int* nbr
 
 // ---- batched Taylor: many trajectories in one persistent launch ---------------------------
 constexpr int kMaxBatch = 128;  // trajectories per launch (the descriptors travel as kernel parameters)
+constexpr int kMaxBatchStreams = 64;
 // batches whose every evolving trajectory has room for at least this many states step their
 // Taylor series through the single-trajectory kernel, one launch per trajectory
 constexpr int64_t kBatchSingleCap = PACES_BATCH_SINGLE_CAP;

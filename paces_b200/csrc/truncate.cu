@@ -632,13 +632,13 @@ template <int NW, int WK, int WKS>
 int launch_truncate_t(const ModelDev& m, const uint64_t* x_keys, const int* x_blk, const void* psi, void* scratch,
                       int64_t maxstates, int shuffle, uint64_t seed, uint64_t step, const TruncWs& ws,
                       uint64_t* out_keys, int* out_blk, int64_t out_cap, float* out_w, int* n_tied_out, int* n_kept_out,
-                      int* status, int num_sms, int at_once, cudaStream_t st) {
+                      int* status, int num_sms, int sel_sms, cudaStream_t st) {
     constexpr bool kStore = WKS != WK;
     const void* src = kStore ? scratch : psi;
     const int g = grid_for(ws.cap, 1024, num_sms * 4);  // streaming passes of the tie shuffle
     {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid_for(ws.cap, kSelThreads * 2, max(num_sms / at_once, 1)));
+        cfg.gridDim = dim3(grid_for(ws.cap, kSelThreads * 2, sel_sms));
         cfg.blockDim = dim3(kSelThreads);
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
@@ -670,11 +670,11 @@ template <int NW>
 int dispatch_prec(bool c64, const ModelDev& m, const uint64_t* x_keys, const int* x_blk,
                   const void* psi, const double* weights, void* scratch, int64_t maxstates, int shuffle, uint64_t seed,
                   uint64_t step, const TruncWs& ws, uint64_t* out_keys, int* out_blk, int64_t out_cap,
-                  float* out_w, int* n_tied_out, int* n_kept_out, int* status, int num_sms, int at_once, cudaStream_t st) {
+                  float* out_w, int* n_tied_out, int* n_kept_out, int* status, int num_sms, int sel_sms, cudaStream_t st) {
 #define PACES_TRUNC_LAUNCH(WK, WKS, SRC)                                                                     \
     return launch_truncate_t<NW, WK, WKS>(m, x_keys, x_blk, SRC, scratch, maxstates, shuffle, seed, step, ws, \
                                           out_keys, out_blk, out_cap, out_w, n_tied_out, n_kept_out, status,  \
-                                          num_sms, at_once, st)
+                                          num_sms, sel_sms, st)
     if (weights) PACES_TRUNC_LAUNCH(2, 2, weights);
     if (c64) {
         if (scratch) PACES_TRUNC_LAUNCH(1, stored_kind(1), psi);
@@ -690,13 +690,13 @@ int dispatch_prec(bool c64, const ModelDev& m, const uint64_t* x_keys, const int
 int launch_truncate(int nw, bool c64, const ModelDev& m, const uint64_t* x_keys, const int* x_blk,
                     const void* psi, const double* weights, void* scratch, int64_t maxstates, int shuffle, uint64_t seed,
                     uint64_t step, const TruncWs& ws, uint64_t* out_keys, int* out_blk, int64_t out_cap, float* out_w,
-                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, int at_once, cudaStream_t st,
+                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, int sel_sms, cudaStream_t st,
                     bool cleared) {
     if (!cleared && cudaMemsetAsync(ws.hist, 0, kTruncHistBytes, st) != cudaSuccess) return PACES_ERR_CUDA;
 #define PACES_TRUNC_CASE(N)                                                                       \
     case N:                                                                                       \
         return dispatch_prec<N>(c64, m, x_keys, x_blk, psi, weights, scratch, maxstates, shuffle, seed, step, ws, \
-                                out_keys, out_blk, out_cap, out_w, n_tied_out, n_kept_out, status, num_sms, at_once, st);
+                                out_keys, out_blk, out_cap, out_w, n_tied_out, n_kept_out, status, num_sms, sel_sms, st);
     switch (nw) {
         PACES_TRUNC_CASE(1)
         PACES_TRUNC_CASE(2)

@@ -50,13 +50,13 @@ inline int trunc_launches(bool shuffle) { return 2 + (shuffle ? 16 : 0); }
 // out_w (optional, out_cap + 1 floats): the ranked weight (|psi|) of every kept state in the
 // new basis' order, and at out_w[out_cap] the cut -- the weight of the smallest kept state, 0
 // when nothing was dropped.
-// at_once: truncations that may run at the same time on this GPU; each takes its share of the
-// SMs for the launch whose blocks wait for one another, so all of them fit together.
+// sel_sms: SMs that the launch whose blocks wait for one another may take; truncations that may
+// run at the same time on this GPU take no more than all of them together.
 // cleared: the caller's last kernel has zeroed ws.hist (kTruncHistBytes)
 int launch_truncate(int nw, bool c64, const ModelDev& m, const uint64_t* x_keys, const int* x_blk,
                     const void* psi, const double* weights, void* scratch, int64_t maxstates, int shuffle, uint64_t seed,
                     uint64_t step, const TruncWs& ws, uint64_t* out_keys, int* out_blk, int64_t out_cap, float* out_w,
-                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, int at_once, cudaStream_t st,
+                    int* n_tied_out, int* n_kept_out, int* status, int num_sms, int sel_sms, cudaStream_t st,
                     bool cleared = false);
 
 }  // namespace paces
