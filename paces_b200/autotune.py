@@ -69,7 +69,7 @@ def bps_candidates(t: nat.Tuning):
 
 
 # bumped when the kernels' tiling changes, so that choices cached for other tiles are not reused
-CACHE_LAYOUT = 2
+CACHE_LAYOUT = 3
 
 
 def _key(eng, states):
