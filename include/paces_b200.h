@@ -263,8 +263,10 @@ int paces_lanczos(paces_ctx *ctx, const paces_basis *basis, const paces_hmat *h,
  * wait_limit_ns (0 = the default 2 s, at most 2 s) bounds each grid-barrier wait of this
  * context's Taylor and scaling-and-squaring kernels; skip_barrier_block >= 0 makes that block
  * give up at its first grid barrier without arriving, so every other block's wait runs out
- * (-1 = off); the Lanczos kernel's grid barriers obey the same hooks.  Results are
- * unaffected while the hooks are off. */
+ * (-1 = off); the Lanczos kernel's grid barriers obey the same hooks, and so do the
+ * truncation's selection in paces_truncate(_weighted) and in a step that does not propagate (a
+ * step that does takes the hooks in its propagation).  Results are unaffected while the hooks
+ * are off. */
 int paces_set_test_hooks(paces_ctx *ctx, uint64_t wait_limit_ns, int32_t skip_barrier_block);
 /* Stage timing (no counterpart in the reference, which only prints wall-clock times):
  * with profiling on, paces_step records CUDA events between its stages, and

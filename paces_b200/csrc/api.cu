@@ -28,7 +28,7 @@ struct paces_ctx {
     int profiling;  // record stage events in paces_step
     cudaEvent_t ev[8];
     unsigned long long launches;  // kernels launched by paces_step since creation
-    uint64_t test_wait_ns;   // test hook: grid-barrier wait limit of the Taylor kernels (0: kWaitLimitNs)
+    uint64_t test_wait_ns;   // test hook: grid-barrier wait limit of this context's kernels (0: kWaitLimitNs)
     int test_skip_block;     // test hook: block that skips its grid-barrier arrival (-1: none)
     char err[512];
 };
@@ -192,8 +192,11 @@ MergeWs merge_ws(const paces_ctx* c, const Layout& l, void* ws, int at_once = 1)
     return w;
 }
 
-TruncWs trunc_ws(const Layout& l, void* ws) {
+// hooked: the context's test hooks apply
+TruncWs trunc_ws(const paces_ctx* c, const Layout& l, void* ws, bool hooked) {
     TruncWs w;
+    w.wait_ns = hooked && c->test_wait_ns ? c->test_wait_ns : kWaitLimitNs;
+    w.skip_block = hooked ? c->test_skip_block : -1;
     w.hist = at<unsigned>(ws, l.t_hist);
     w.cand = at<unsigned long long>(ws, l.t_cand);
     w.cand_idx = at<int>(ws, l.t_cand_idx);
@@ -456,7 +459,7 @@ int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks, int sel_s
     void* wscratch = weights ? nullptr : at<void>(ws, l.v_TA);
     PACES_CHECK_LAUNCH(c, launch_truncate(c->nw, c64, c->m, p.old_b->keys, p.old_b->blk, p.old_psi, weights, wscratch,
                                           prm->maxstates,
-                                          prm->shuffle, prm->shuffle_seed, prm->step_index, trunc_ws(l, ws), p.A.keys,
+                                          prm->shuffle, prm->shuffle_seed, prm->step_index, trunc_ws(c, l, ws, !prm->evolve), p.A.keys,
                                           p.A.blk, p.A.cap, at<float>(ws, l.aw), &rec->n_tied, &rec->n_select, status, c->num_sms, sel_sms,
                                           st, true),
                        "step/truncate");
@@ -976,7 +979,7 @@ int paces_truncate(paces_ctx* c, const paces_basis* in, const void* psi, int64_t
     const Layout l = fit_layout(c, ws_bytes);
     if (in->cap > l.cap) return fail(c, PACES_ERR_CAPACITY, "workspace holds %lld states, input basis %lld", (long long)l.cap, (long long)in->cap);
     PACES_CHECK_LAUNCH(c, launch_truncate(c->nw, c->precision == PACES_C64, c->m, in->keys, in->blk, psi, nullptr,
-                                          at<void>(ws, l.v_TA), maxstates, shuffle, shuffle_seed, step_index, trunc_ws(l, ws), out->keys,
+                                          at<void>(ws, l.v_TA), maxstates, shuffle, shuffle_seed, step_index, trunc_ws(c, l, ws, true), out->keys,
                                           out->blk, out->cap, nullptr, nullptr, nullptr, c->d_status, c->num_sms, c->num_sms,
                                           reinterpret_cast<cudaStream_t>(stream)),
                        "truncate");
@@ -990,7 +993,7 @@ int paces_truncate_weighted(paces_ctx* c, const paces_basis* in, const double* w
     const Layout l = fit_layout(c, ws_bytes);
     if (in->cap > l.cap) return fail(c, PACES_ERR_CAPACITY, "workspace holds %lld states, input basis %lld", (long long)l.cap, (long long)in->cap);
     PACES_CHECK_LAUNCH(c, launch_truncate(c->nw, c->precision == PACES_C64, c->m, in->keys, in->blk, nullptr, weights,
-                                          nullptr, maxstates, shuffle, shuffle_seed, step_index, trunc_ws(l, ws), out->keys,
+                                          nullptr, maxstates, shuffle, shuffle_seed, step_index, trunc_ws(c, l, ws, true), out->keys,
                                           out->blk, out->cap, nullptr, nullptr, nullptr, c->d_status, c->num_sms, c->num_sms,
                                           reinterpret_cast<cudaStream_t>(stream)),
                        "truncate_weighted");

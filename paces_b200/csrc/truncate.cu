@@ -247,7 +247,7 @@ trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restr
     const int64_t S = x_blk[L];
     const bool all = S <= maxstates;
     if (blockIdx.x == 0 && tid < SEL_WORDS) {
-        // until the selection is known: nothing to write (a wait that runs out leaves it so)
+        // until the selection is known: nothing to write
         long long v = 0;
         if (tid == SEL_ALL) v = 1;
         if (all && tid == SEL_S) v = S;
@@ -257,6 +257,13 @@ trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restr
     const int64_t nch = (S + kTruncChunk - 1) / kTruncChunk;
     const int64_t c0 = nch * blockIdx.x / gridDim.x, c1 = nch * (blockIdx.x + 1) / gridDim.x;  // this block's chunks
     unsigned gen = 0;
+    // A block whose wait runs out says so: the others may have gone on and finished, but without its
+    // chunks' prefixes the compaction would place states wrongly, so it writes none.
+    auto grid_wait = [&]() {
+        const bool ok = grid_barrier(ws.barrier, gridDim.x, gen, status, ws.wait_ns, int(blockIdx.x) == ws.skip_block);
+        if (!ok && tid == 0) ws.barrier[kTruncGaveUp] = 1u;
+        return ok;
+    };
     unsigned long long lo = 0, width = ~0ull;
     long long need = maxstates, count = S;
     const void* src = psi;
@@ -293,7 +300,7 @@ trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restr
         unsigned* gh = ws.hist + (round % 3) * 4096;
         for (int b = tid; b < 4096; b += kSelThreads)
             if (h[b]) atomicAdd(&gh[b], h[b]);
-        if (!grid_barrier(ws.barrier, gridDim.x, gen, status)) return;
+        if (!grid_wait()) return;
         constexpr int per = 4096 / kSelThreads;
         unsigned hb[per];
 #pragma unroll
@@ -331,7 +338,7 @@ trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restr
             na += __popc(__ballot_sync(0xffffffffu, v && !in));
             if (list) {
                 if (in) {
-                    const unsigned slot = atomicAdd(ws.barrier + 1, 1u);
+                    const unsigned slot = atomicAdd(ws.barrier + kTruncListed, 1u);
                     if (slot < kSelCand && slot < ws.cap) {
                         ws.cand[slot] = k[u];
                         ws.cand_idx[slot] = int(c * kTruncChunk + 32 * u + lane);
@@ -349,7 +356,7 @@ trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restr
     });
     long long ties = count;
     if (list) {
-        if (!grid_barrier(ws.barrier, gridDim.x, gen, status)) return;
+        if (!grid_wait()) return;
         // the need-th largest of the listed weights, 12 bits a round
         const int n = int(count);
         constexpr int kMine = kSelCand / kSelThreads, per = 4096 / kSelThreads;
@@ -398,7 +405,7 @@ trunc_threshold_kernel(int L, const int* __restrict__ x_blk, const void* __restr
     // exclusive prefixes: the blocks' totals, then this block's chunks
     __syncthreads();
     if (tid == 0) ws.block_sum[blockIdx.x] = s_own;
-    if (!grid_barrier(ws.barrier, gridDim.x, gen, status)) return;
+    if (!grid_wait()) return;
     unsigned long long before, total;
     block_prefix(tid < blockIdx.x ? __ldcg(ws.block_sum + tid) : 0ull, s_sum, before);
     for (int64_t c = c0; c < c1; c += kSelThreads) {
@@ -538,8 +545,9 @@ __global__ void __launch_bounds__(256, NW <= 2 ? 4 : (NW <= 4 ? 3 : 2)) trunc_wr
     const int L = m.L;
     for (int i = threadIdx.x; i <= L; i += blockDim.x) s_blk[i] = x_blk[i];
     __syncthreads();
-    const int64_t S = ws.sel[SEL_S];
-    const bool all = ws.sel[SEL_ALL] != 0;
+    const bool gave_up = ws.barrier[kTruncGaveUp] != 0;  // nothing is written
+    const int64_t S = gave_up ? 0 : ws.sel[SEL_S];
+    const bool all = gave_up || ws.sel[SEL_ALL] != 0;
     const unsigned long long vstar = (unsigned long long)ws.sel[SEL_W + 0];
     const long long skip_ties = ws.sel[SEL_TIES] - ws.sel[SEL_W + 2];  // tied states dropped (the lowest indices)
     const bool shuf = ws.sel[SEL_SHUFFLE] != 0;
@@ -609,7 +617,7 @@ __global__ void __launch_bounds__(256, NW <= 2 ? 4 : (NW <= 4 ? 3 : 2)) trunc_wr
     __syncthreads();
     if (threadIdx.x != 0) return;
     __threadfence();
-    if (atomicAdd(ws.barrier + 2, 1u) != gridDim.x - 1) return;
+    if (atomicAdd(ws.barrier + kTruncDone, 1u) != gridDim.x - 1) return;
     __threadfence();
     // the cut: |psi| of the smallest kept state when states were dropped, else 0
     if (out_w) out_w[out_cap] = all ? 0.f : float(__longlong_as_double((long long)vstar));

@@ -22,14 +22,20 @@ namespace paces {
 
 struct TruncWs {
     unsigned* hist;              // [3][4096] radix histograms in rotation
-    unsigned* barrier;           // behind them: grid barrier, listed states, blocks done
+    unsigned* barrier;           // behind them: the grid barrier and the counters below
     unsigned long long* cand;    // [cap] candidate weight bits (or hashes)
     int* cand_idx;               // [cap]
     long long* sel;              // selection state, see truncate.cu
     unsigned long long* block_sum;   // [1024] the selection's blocks: counts of their chunks
     unsigned long long* chunk;       // [trunc_chunks_cap(cap)] counts, then prefixes of the chunks
     int64_t cap;
+    uint64_t wait_ns;            // grid-barrier wait limit (kWaitLimitNs unless a test shortens it)
+    int skip_block;              // test hook: this block skips its first grid-barrier arrival (-1: none)
 };
+// words of TruncWs.barrier
+constexpr int kTruncListed = 1;  // states listed for the last bin
+constexpr int kTruncDone = 2;    // blocks of the compaction done
+constexpr int kTruncGaveUp = 3;  // a block of the selection gave up waiting
 constexpr size_t kTruncHistBytes = (3 * 4096 + 16) * 4;  // histograms and counters, zeroed per truncation
 
 constexpr int kTruncChunk = 256;  // states a warp of the compaction takes at a time
