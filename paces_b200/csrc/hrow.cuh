@@ -9,10 +9,10 @@
 // rounds every product and sum separately (no fused multiply-add), so it reproduces
 // the reference arithmetic row by row.
 //
-// The rows are branch-free: every neighbour load is issued (an absent neighbour re-reads
-// the row's own element, already in flight, and its term is discarded by a select), so
-// the five loads of a row -- and of several rows handled by one thread -- are in flight
-// together without funnelling the absent ones onto one hot cache line.
+// The rows are branch-free, so the five loads of a row -- and of several rows handled by one
+// thread -- are in flight together.  An absent neighbour is a load left out by its predicate
+// (see `neighbour`); complex64 chains and couplings re-read the row's own element instead,
+// already in flight, under a zero coefficient.
 #pragma once
 
 #include "common.cuh"
@@ -36,6 +36,15 @@ __device__ __forceinline__ int4 load_nbr(const int* __restrict__ nbr, int64_t r)
     return __ldg(reinterpret_cast<const int4*>(nbr) + r);
 }
 
+// x[idx], or zero for an absent neighbour (idx < 0).  A coefficient of zero would not do: times an
+// infinite element of the row itself it is a NaN where the row's sum is infinite.
+template <class C>
+__device__ __forceinline__ C neighbour(const C* __restrict__ x, int idx) {
+    C v{};
+    if (idx >= 0) v = __ldcg(x + idx);
+    return v;
+}
+
 // The same, read once per sweep of a table larger than L2: not kept in the caches.
 __device__ __forceinline__ int4 ldcs_nbr(const int* __restrict__ nbr, int64_t r) {
     return __ldcs(reinterpret_cast<const int4*>(nbr) + r);
@@ -47,17 +56,14 @@ template <class P>
 __device__ __forceinline__ double2 h_row_c128_nb(const P& m, const double* sq, int64_t r, int4 nb, uint32_t meta,
                                                  double2 xr, const double2* __restrict__ x) {
     const int n = int((meta >> 8) & 0xffu);
-    const double2 xa = __ldcg(x + (nb.x >= 0 ? nb.x : r));
-    const double2 xb = __ldcg(x + (nb.y >= 0 ? nb.y : r));
-    const double2 xd = __ldcg(x + (nb.z >= 0 ? nb.z : r));
-    const double2 xu = __ldcg(x + (nb.w >= 0 ? nb.w : r));
+    const double2 xa = neighbour(x, nb.x), xb = neighbour(x, nb.y);
+    const double2 xd = neighbour(x, nb.z), xu = neighbour(x, nb.w);
     const double d = diag_value(m, meta);
     // the CSR row sums hop and coupling pairs by themselves; a two-term sum does not depend on
     // the column order, and an absent neighbour's zero product leaves the sum as it is
-    const double ja = nb.x >= 0 ? m.J : 0.0, jb = nb.y >= 0 ? m.J : 0.0;
-    const double cd = nb.z >= 0 ? sq[n] : 0.0, cu = nb.w >= 0 ? sq[n + 1] : 0.0;
-    const double hx = __dadd_rn(__dmul_rn(ja, xa.x), __dmul_rn(jb, xb.x));
-    const double hy = __dadd_rn(__dmul_rn(ja, xa.y), __dmul_rn(jb, xb.y));
+    const double cd = sq[n], cu = sq[n + 1];
+    const double hx = __dadd_rn(__dmul_rn(m.J, xa.x), __dmul_rn(m.J, xb.x));
+    const double hy = __dadd_rn(__dmul_rn(m.J, xa.y), __dmul_rn(m.J, xb.y));
     const double vx = __dadd_rn(__dmul_rn(cd, xd.x), __dmul_rn(cu, xu.x));
     const double vy = __dadd_rn(__dmul_rn(cd, xd.y), __dmul_rn(cu, xu.y));
     return make_double2(__dadd_rn(__dadd_rn(__dmul_rn(d, xr.x), hx), vx), __dadd_rn(__dadd_rn(__dmul_rn(d, xr.y), hy), vy));
@@ -116,10 +122,9 @@ __device__ __forceinline__ int hop_index(const ModelDev& m, int64_t r, int4 nb, 
 }
 //
 // GEO is the number of lattice dimensions: a term has one channel per dimension.  A term's
-// indices are read and its gathers issued before its sum, an absent neighbour re-reading the
-// row's own element under a zero coefficient (which leaves the sum as it is); the sum visits
-// the lower neighbours from the largest distance and the upper ones from the smallest, the
-// column order.  With the channels a runtime loop the gathers waited for one another (866K
+// indices are read and its gathers issued before its sum, an absent neighbour being zero (which
+// leaves the sum as it is); the sum visits the lower neighbours from the largest distance and
+// the upper ones from the smallest, the column order.  With the channels a runtime loop the gathers waited for one another (866K
 // rows of a square lattice with both terms, complex128: 41 us a Taylor sweep, now 21); three
 // dimensions unrolled for every model spilled (47 us).
 template <int GEO>
@@ -141,8 +146,7 @@ template <int GEO>
 __device__ __forceinline__ double2 h_row_c128_geo(const ModelDev& m, const double* sq, int64_t r, int4 nb, uint32_t meta,
                                                   double2 xr, const double2* __restrict__ x) {
     const int n = int((meta >> 8) & 0xffu);
-    const double2 xd = __ldcg(x + (nb.z >= 0 ? nb.z : r));
-    const double2 xu = __ldcg(x + (nb.w >= 0 ? nb.w : r));
+    const double2 xd = neighbour(x, nb.z), xu = neighbour(x, nb.w);
     const double d = diag_value(m, meta);
     double2 y = make_double2(__dmul_rn(d, xr.x), __dmul_rn(d, xr.y));
 #pragma unroll
@@ -154,21 +158,20 @@ __device__ __forceinline__ double2 h_row_c128_geo(const ModelDev& m, const doubl
         double2 vl[GEO], vu[GEO];
 #pragma unroll
         for (int k = 0; k < GEO; ++k) {
-            vl[k] = __ldcg(x + (lo[k] >= 0 ? lo[k] : r));
-            vu[k] = __ldcg(x + (up[k] >= 0 ? up[k] : r));
+            vl[k] = neighbour(x, lo[k]);
+            vu[k] = neighbour(x, up[k]);
         }
         double2 hs = make_double2(0.0, 0.0);
-        auto add = [&](int idx, const double2& v) {
-            const double c = idx >= 0 ? Jt : 0.0;
-            hs = make_double2(__dadd_rn(hs.x, __dmul_rn(c, v.x)), __dadd_rn(hs.y, __dmul_rn(c, v.y)));
+        auto add = [&](const double2& v) {
+            hs = make_double2(__dadd_rn(hs.x, __dmul_rn(Jt, v.x)), __dadd_rn(hs.y, __dmul_rn(Jt, v.y)));
         };
 #pragma unroll
-        for (int k = GEO - 1; k >= 0; --k) add(lo[k], vl[k]);
+        for (int k = GEO - 1; k >= 0; --k) add(vl[k]);
 #pragma unroll
-        for (int k = 0; k < GEO; ++k) add(up[k], vu[k]);
+        for (int k = 0; k < GEO; ++k) add(vu[k]);
         y = make_double2(__dadd_rn(y.x, hs.x), __dadd_rn(y.y, hs.y));
     }
-    const double cd = nb.z >= 0 ? sq[n] : 0.0, cu = nb.w >= 0 ? sq[n + 1] : 0.0;
+    const double cd = sq[n], cu = sq[n + 1];
     const double vx = __dadd_rn(__dmul_rn(cd, xd.x), __dmul_rn(cu, xu.x));
     const double vy = __dadd_rn(__dmul_rn(cd, xd.y), __dmul_rn(cu, xu.y));
     return make_double2(__dadd_rn(y.x, vx), __dadd_rn(y.y, vy));
@@ -191,18 +194,17 @@ __device__ __forceinline__ float2 h_row_c64_geo(const ModelDev& m, const float* 
         float2 vl[GEO], vu[GEO];
 #pragma unroll
         for (int k = 0; k < GEO; ++k) {
-            vl[k] = __ldcg(x + (lo[k] >= 0 ? lo[k] : r));
-            vu[k] = __ldcg(x + (up[k] >= 0 ? up[k] : r));
+            vl[k] = neighbour(x, lo[k]);
+            vu[k] = neighbour(x, up[k]);
         }
-        auto add = [&](int idx, const float2& v) {
-            const float c = idx >= 0 ? Jt : 0.f;
-            y.x = fmaf(c, v.x, y.x);
-            y.y = fmaf(c, v.y, y.y);
+        auto add = [&](const float2& v) {
+            y.x = fmaf(Jt, v.x, y.x);
+            y.y = fmaf(Jt, v.y, y.y);
         };
 #pragma unroll
-        for (int k = GEO - 1; k >= 0; --k) add(lo[k], vl[k]);
+        for (int k = GEO - 1; k >= 0; --k) add(vl[k]);
 #pragma unroll
-        for (int k = 0; k < GEO; ++k) add(up[k], vu[k]);
+        for (int k = 0; k < GEO; ++k) add(vu[k]);
     }
     const float cd = nb.z >= 0 ? sq[n] : 0.f, cu = nb.w >= 0 ? sq[n + 1] : 0.f;
     y.x = fmaf(cd, xd.x, y.x);
