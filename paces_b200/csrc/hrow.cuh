@@ -69,13 +69,6 @@ __device__ __forceinline__ double2 h_row_c128_nb(const P& m, const double* sq, i
     return make_double2(__dadd_rn(__dadd_rn(__dmul_rn(d, xr.x), hx), vx), __dadd_rn(__dadd_rn(__dmul_rn(d, xr.y), hy), vy));
 }
 
-template <class P>
-__device__ __forceinline__ double2 h_row_c128(const P& m, const double* sq, int64_t r,
-                                              const int* __restrict__ nbr, uint32_t meta,
-                                              const double2* __restrict__ x) {
-    return h_row_c128_nb(m, sq, r, load_nbr(nbr, r), meta, __ldcg(x + r), x);
-}
-
 // y = (H x)[r] in complex64 with fp32 accumulation.  sq[k] = float(sqrt(k) * g).
 template <class P>
 __device__ __forceinline__ float2 h_row_c64_nb(const P& m, const float* sq, float J, int64_t r, int4 nb,
@@ -98,13 +91,6 @@ __device__ __forceinline__ float2 h_row_c64_nb(const P& m, const float* sq, floa
     y.x = fmaf(cu, xu.x, y.x);
     y.y = fmaf(cu, xu.y, y.y);
     return y;
-}
-
-template <class P>
-__device__ __forceinline__ float2 h_row_c64(const P& m, const float* sq, float J, int64_t r,
-                                            const int* __restrict__ nbr, uint32_t meta,
-                                            const float2* __restrict__ x) {
-    return h_row_c64_nb(m, sq, J, r, load_nbr(nbr, r), meta, __ldcg(x + r), x);
 }
 
 // ---- lattices with several hopping channels (ModelDev::nhop > 1) ---------------------------

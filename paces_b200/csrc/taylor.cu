@@ -49,7 +49,7 @@ constexpr int kTWarps = kTThreads / 32;
 // GEO: 0 the chain, otherwise the dimensions of a lattice with several hopping channels (h_row_*_geo).
 template <bool C64, bool STREAM, int GEO>
 __global__ void __launch_bounds__(kTThreads, STREAM ? (C64 ? 3 : 2) : (C64 ? 4 : 3))
-taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ nbr, int64_t cap,
+taylor_kernel(ModelDev m, const int* __restrict__ blk, const int* __restrict__ nbr,
               const uint32_t* __restrict__ meta, const void* v_in, void* res_out, TaylorWs ws,
               double dt, int m_star, double tol, TaylorOut out, int* status) {
     using C = typename std::conditional<C64, float2, double2>::type;
@@ -238,10 +238,10 @@ int occupancy_any(bool c64, int variant, int geo) {
 }
 
 template <bool C64, bool STREAM, int GEO>
-cudaError_t launch_one(const cudaLaunchConfig_t& cfg, const ModelDev& m, const int* blk, const int* nbr, int64_t cap,
+cudaError_t launch_one(const cudaLaunchConfig_t& cfg, const ModelDev& m, const int* blk, const int* nbr,
                        const uint32_t* meta, const void* v_in, void* res, const TaylorWs& ws, double dt, int m_star,
                        double tol, const TaylorOut& out, int* status) {
-    return cudaLaunchKernelEx(&cfg, taylor_kernel<C64, STREAM, GEO>, m, blk, nbr, cap, meta, v_in, res, ws, dt, m_star,
+    return cudaLaunchKernelEx(&cfg, taylor_kernel<C64, STREAM, GEO>, m, blk, nbr, meta, v_in, res, ws, dt, m_star,
                               tol, out, status);
 }
 
@@ -278,10 +278,9 @@ int launch_taylor(bool c64, const ModelDev& m, const int* blk, const int* nbr, i
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int64_t cap = nbr_cap;
     cudaError_t e;
 #define PACES_TAYLOR_ONE(C, B, G) \
-    launch_one<C, B, G>(cfg, m, blk, nbr, cap, meta, v_in, res, ws, dt, m_star, tol, out, status)
+    launch_one<C, B, G>(cfg, m, blk, nbr, meta, v_in, res, ws, dt, m_star, tol, out, status)
 #define PACES_TAYLOR_GEO(C, B)                                             \
     (geo == 0 ? PACES_TAYLOR_ONE(C, B, 0)                                  \
               : (geo == 1 ? PACES_TAYLOR_ONE(C, B, 1)                      \

@@ -118,11 +118,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(mbar)
                  : "memory");
 }
-// order this thread's earlier generic-proxy global accesses (and those it synchronised
-// with) before its later async-proxy (bulk copy) accesses
-__device__ __forceinline__ void fence_proxy_async_global() {
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-}
 
 }  // namespace tc
 }  // namespace paces
