@@ -240,8 +240,8 @@ int64_t self_flag_cap(const paces_ctx* c, const Layout& l) {
     return l.cap * int64_t(c->precision == PACES_C64 ? 8 : 16);
 }
 
-// The caller's Krylov workspace of the Lanczos step: order+1 vectors, two w buffers, the
-// per-block partial sums and the barrier words.
+// The caller's Krylov workspace of the Lanczos step: the columns 1 .. order, the per-block
+// partial sums and the barrier words.
 struct KrylovLayout {
     size_t u, partials, barrier, total;
     int max_grid;
@@ -455,7 +455,7 @@ int step_front(paces_ctx* c, StepPlan& p, cudaStream_t st, bool marks, int sel_s
                            "step/weights");
         weights = w;
     }
-    // without look-ahead weights the same buffer holds |psi| after the first radix round
+    // without look-ahead weights the same buffer holds |psi| after the selection's first pass
     void* wscratch = weights ? nullptr : at<void>(ws, l.v_TA);
     PACES_CHECK_LAUNCH(c, launch_truncate(c->nw, c64, c->m, p.old_b->keys, p.old_b->blk, p.old_psi, weights, wscratch,
                                           prm->maxstates,
@@ -1471,9 +1471,10 @@ int paces_batch_step(paces_batch* b, const paces_batch_item* items, int32_t n, p
     mark(1);
     // 2. the Taylor series.  Batches of large trajectories (every evolving one with room for at
     //    least kBatchSingleCap states) run them one after the other through the single-trajectory
-    //    kernel (0.85 against 0.61 of HBM on 64M-row trajectories, measured before both kernels
-    //    streamed rows through registers); otherwise one persistent launch serves all.  Both give
-    //    the same results.  Test hooks on the batch keep the batched launch.
+    //    kernel, which streams long row ranges faster: complex64, two trajectories of 58.8M rows
+    //    10.5 ms against 13.3, two of 15.2M rows 2.66 against 3.54.  Small ones go through one
+    //    persistent launch (eight of 0.3M rows: 0.25 ms against 0.53).  Both give the same results.
+    //    Test hooks on the batch keep the batched launch.
     bool per_item = n_evolve > 0 && b->test_wait_ns == 0 && b->test_skip_block < 0;
     for (int i = 0; i < n && per_item; ++i)
         if (items[i].params->evolve && plans[i].new_b->cap < kBatchSingleCap) per_item = false;

@@ -111,7 +111,7 @@ __device__ __forceinline__ int hop_index(const ModelDev& m, int64_t r, int4 nb, 
 // indices are read and its gathers issued before its sum, an absent neighbour being zero (which
 // leaves the sum as it is); the sum visits the lower neighbours from the largest distance and
 // the upper ones from the smallest, the column order.  With the channels a runtime loop the gathers waited for one another (866K
-// rows of a square lattice with both terms, complex128: 41 us a Taylor sweep, now 21); three
+// rows of a square lattice with both terms, complex128: 41 us a Taylor sweep, now 20); three
 // dimensions unrolled for every model spilled (47 us).
 template <int GEO>
 __device__ __forceinline__ void load_hops(const ModelDev& m, int t, int64_t r, int4 nb, int (&lo)[GEO], int (&up)[GEO]) {

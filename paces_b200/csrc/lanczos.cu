@@ -20,7 +20,7 @@
 // and storing it as well cost a vector written per A sweep.  A warp takes rows in units of 64, two
 // per lane, and the next unit's loads are under way while this unit's gathers wait on L2.
 // (A sweep that stored q_i and w, rows a grid stride apart, loads of the next row only after
-// this one's gathers: 337 us for 13 vectors of 825K complex128 rows; 276 now, with the sums and the
+// this one's gathers: 337 us for 13 vectors of 825K complex128 rows; 270 now, with the sums and the
 // small exponential below.)
 // The partial sums are fp64 (complex64 vectors too) and every block adds the per-block
 // partials in the same order, so all blocks hold bit-identical alpha and beta and take the
@@ -50,7 +50,7 @@ static_assert(kKrylovMax <= 64, "the small exponential holds two rows per lane o
 // them, publishes the block's partial in ws.partials[parity], passes the barrier and adds all
 // blocks' partials -- in the same order in every block, so the sums agree in every bit.  The
 // result is in fin[0..NV) for every thread; false when the barrier timed out.  (With the partials
-// added by the whole block, two more block barriers a sum: 285 us a launch of 12 vectors, now 276.)
+// added by the whole block, two more block barriers a sum: 9 us more of a launch of 12 vectors.)
 template <int NV>
 __device__ bool grid_sum(double v[NV], const LanczosWs& ws, int parity, unsigned& gen, int* status,
                          double (*red)[kLWarps], double* fin) {

@@ -26,7 +26,7 @@ __host__ __device__ constexpr int round_bits(int r) { return r < 5 ? 12 : 4; }
 
 // The ranked weight of state i: WK 0 = |psi| of complex128 amplitudes, 1 = |psi| of
 // complex64 amplitudes, 2 = precomputed non-negative fp64 weights (the look-ahead
-// weighting, or |psi| of complex128 amplitudes stored by the first radix round), 3 = |psi|
+// weighting, or |psi| of complex128 amplitudes stored by the first pass), 3 = |psi|
 // of complex64 amplitudes stored as fp32 by the first round (exact: hypotf's result,
 // widened like WK 1 widens it).  Non-negative doubles order like their bit patterns.  The
 // load and the conversion are separate so that loops can issue several loads before the

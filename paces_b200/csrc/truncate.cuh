@@ -51,7 +51,7 @@ inline int trunc_launches(bool shuffle) { return 2 + (shuffle ? 16 : 0); }
 // weights (optional, one non-negative double per state): rank by these instead of |psi|
 // (the look-ahead weighting, lookahead.cu).
 // scratch (optional, without weights: 4 bytes per state for complex64, 8 for complex128):
-// the first radix round stores |psi| there and the later passes read it instead of the
+// the selection's first pass stores |psi| there and the later passes read it instead of the
 // amplitudes, so |psi| is computed once per state.
 // out_w (optional, out_cap + 1 floats): the ranked weight (|psi|) of every kept state in the
 // new basis' order, and at out_w[out_cap] the cut -- the weight of the smallest kept state, 0
