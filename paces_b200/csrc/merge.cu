@@ -818,7 +818,7 @@ __host__ __device__ constexpr size_t tile_blocks_offset(int tmax, int mode) {
             size_t(tmax) * (mode == MERGE_EXPAND_SPLIT ? 8 : 6) + 3) & ~size_t(3);
 }
 template <int NW>
-size_t tile_smem_bytes(int tmax, int mode, int L) {
+constexpr size_t tile_smem_bytes(int tmax, int mode, int L) {
     return tile_blocks_offset<NW>(tmax, mode) + size_t(2) * (L + 1) * sizeof(int);
 }
 
@@ -1172,7 +1172,11 @@ void launch_tile(int tmax, const ModelDev& m, const uint64_t* X, const uint64_t*
                  const MergeOut& out, int* ceiling_out, int ceiling_add, int* status, int num_sms, cudaStream_t st) {
     const size_t smem = tile_smem_bytes<NW>(tmax, MODE, m.L);
     auto kfn = merge_tile_kernel<NW, MODE>;
-    cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    // The limit is the kernel's, not the launch's, and threads launch it with different tiles at the
+    // same time: every launch sets the same one, the widest tile's on the longest chain.
+    constexpr size_t most = tile_smem_bytes<NW>(merge_tmax(merge_stride(NW)), MODE, kMaxSites);
+    static_assert(most <= 200 * 1024, "a tile fits a block's shared memory");
+    cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most));
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kTileThreads, smem);
     const int grid = num_sms * max(per_sm, 1);
