@@ -599,15 +599,19 @@ template <int NW, bool C64>
 int launch_obs_t(const ModelDev& m, const uint64_t* keys, const int* blk, const int* nbr,
                  int64_t nbr_cap, const uint32_t* meta, const void* psi, int what, double* partials,
                  const ObsTarget& out, int num_sms, cudaStream_t st) {
-    static int grid_e = 0, grid_ex = 0, grid_s = 0, grid_s4 = 0, grid_s2 = 0, grid_sg = 0;
-    if (grid_e == 0) {
-        grid_e = wave_blocks(obs_energy_kernel<C64, false>, num_sms);
-        grid_ex = wave_blocks(obs_energy_kernel<C64, true>, num_sms);
-        grid_sg = wave_blocks(obs_sites_kernel<NW, C64, -1>, num_sms);
-        if constexpr (NW <= 2) grid_s = wave_blocks(obs_sites_kernel<NW, C64, 0>, num_sms);
-        if constexpr (NW <= 4) grid_s4 = wave_blocks(obs_sites_kernel<NW, C64, 4>, num_sms);
-        if constexpr (NW <= 2) grid_s2 = wave_blocks(obs_sites_kernel<NW, C64, 2>, num_sms);
-    }
+    // set by the first thread that comes here, whole before another reads them
+    struct Grids {
+        int e, ex, s = 0, s4 = 0, s2 = 0, sg;
+        explicit Grids(int sms) {
+            e = wave_blocks(obs_energy_kernel<C64, false>, sms);
+            ex = wave_blocks(obs_energy_kernel<C64, true>, sms);
+            sg = wave_blocks(obs_sites_kernel<NW, C64, -1>, sms);
+            if constexpr (NW <= 2) s = wave_blocks(obs_sites_kernel<NW, C64, 0>, sms);
+            if constexpr (NW <= 4) s4 = wave_blocks(obs_sites_kernel<NW, C64, 4>, sms);
+            if constexpr (NW <= 2) s2 = wave_blocks(obs_sites_kernel<NW, C64, 2>, sms);
+        }
+    };
+    static const Grids grids(num_sms);
     const bool energy = (what & PACES_OBS_ENERGY) != 0;
     const bool sites = (what & PACES_OBS_SITES) != 0;
     double* part_e = partials;
@@ -615,11 +619,11 @@ int launch_obs_t(const ModelDev& m, const uint64_t* keys, const int* blk, const 
     int nb_e = 0, nb_s = 0;
     if (energy || !sites) {
         if (m.nhop > 1) {
-            obs_energy_kernel<C64, true><<<grid_ex, kOThreads, 0, st>>>(m, blk, nbr, nbr_cap, meta, psi, part_e);
-            nb_e = grid_ex;
+            obs_energy_kernel<C64, true><<<grids.ex, kOThreads, 0, st>>>(m, blk, nbr, nbr_cap, meta, psi, part_e);
+            nb_e = grids.ex;
         } else {
-            obs_energy_kernel<C64, false><<<grid_e, kOThreads, 0, st>>>(m, blk, nbr, nbr_cap, meta, psi, part_e);
-            nb_e = grid_e;
+            obs_energy_kernel<C64, false><<<grids.e, kOThreads, 0, st>>>(m, blk, nbr, nbr_cap, meta, psi, part_e);
+            nb_e = grids.e;
         }
     }
     if (sites) {
@@ -634,28 +638,28 @@ int launch_obs_t(const ModelDev& m, const uint64_t* keys, const int* blk, const 
         bool done = false;
         if constexpr (NW <= 4) {
             if (uniform && ub == 4) {
-                obs_sites_kernel<NW, C64, 4><<<grid_s4, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
-                nb_s = grid_s4;
+                obs_sites_kernel<NW, C64, 4><<<grids.s4, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
+                nb_s = grids.s4;
                 done = true;
             }
         }
         if constexpr (NW <= 2) {
             if (uniform && ub == 2) {
-                obs_sites_kernel<NW, C64, 2><<<grid_s2, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
-                nb_s = grid_s2;
+                obs_sites_kernel<NW, C64, 2><<<grids.s2, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
+                nb_s = grids.s2;
                 done = true;
             }
         }
         if constexpr (NW <= 2) {
             if (uniform && !done) {
-                obs_sites_kernel<NW, C64, 0><<<grid_s, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
-                nb_s = grid_s;
+                obs_sites_kernel<NW, C64, 0><<<grids.s, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
+                nb_s = grids.s;
                 done = true;
             }
         }
         if (!done) {
-            obs_sites_kernel<NW, C64, -1><<<grid_sg, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
-            nb_s = grid_sg;
+            obs_sites_kernel<NW, C64, -1><<<grids.sg, kOThreads, 0, st>>>(m, keys, blk, meta, psi, part_s, ub, fpw);
+            nb_s = grids.sg;
         }
     }
     if (out.new_blk && !sites) return PACES_ERR_BADARG;  // step_end's block follows the sites'

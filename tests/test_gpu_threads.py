@@ -49,3 +49,44 @@ def test_concurrent_trajectories_equal_themselves_alone():
     for got, want in zip(together, alone):
         assert len(got) == len(want) == 4, (got, want)
         assert got[:3] == want[:3] and torch.equal(got[3], want[3])
+
+
+FIRST_USE = """
+import threading, torch
+from tests import gpu_helpers
+for nchain in (16, 32, 48, 64, 80, 96, 112, 128):  # one to eight key words: kernels of their own
+    for precision in ("c64", "c128"):
+        items = []
+        for _ in range(4):
+            eng = gpu_helpers.engine_for(nchain, 16, 1.0, cap=1 << 12, precision=precision)
+            b, h, _ = eng.assemble(eng.basis_from_ref(gpu_helpers.initial_rows(nchain)))
+            psi = eng.new_vector(b.cap)
+            psi[:b.count()] = 0.5
+            items.append((eng, b, h, psi))
+        torch.cuda.synchronize()
+        gate, out = threading.Barrier(len(items)), [None] * len(items)
+
+        def run(i):
+            eng, b, h, psi = items[i]
+            with torch.cuda.stream(torch.cuda.Stream()):
+                gate.wait()
+                try:
+                    out[i] = eng.observables(b, h, psi)["norm"]
+                except Exception as e:
+                    out[i] = repr(e)
+        threads = [threading.Thread(target=run, args=(i,)) for i in range(len(items))]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert out[0] == out[1] == out[2] == out[3], (nchain, precision, out)
+"""
+
+
+def test_first_observables_of_a_process_on_several_threads():
+    import os
+    import subprocess
+    import sys
+    repo = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", FIRST_USE], cwd=repo, capture_output=True, text=True, timeout=240)
+    assert run.returncode == 0, run.stderr[-2000:]
